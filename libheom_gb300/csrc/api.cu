@@ -348,6 +348,8 @@ struct heomgb_qme {
   heomgb_mlp* term = nullptr;  // learned terminator (not owned); null = plain truncation
   const float2* term_cke = nullptr;  // its set-up tables (TermModel::cke, sgn), in term_arena
   const float* term_sgn = nullptr;
+  const float2* term_rowf = nullptr;  // and TermModel::rowf, isig
+  const float2* term_isig = nullptr;
   TermBuffers diff_tb;       // terminator buffers for calc_diff
   DeviceArena term_arena;
   DeviceArena arena;
@@ -1037,6 +1039,8 @@ TermModel term_model(const heomgb_qme* q) {
   tm.bath_ptr = q->dm.bath_ptr;
   tm.cke = q->term_cke;
   tm.sgn = q->term_sgn;
+  tm.rowf = q->term_rowf;
+  tm.isig = q->term_isig;
   return tm;
 }
 
@@ -2210,6 +2214,7 @@ heomgb_status heomgb_qme_set_terminator(heomgb_qme* q, heomgb_mlp* mlp) {
     DiagInst di = q->dinst;
     q->term_cke = nullptr;
     q->term_sgn = nullptr;
+    q->term_rowf = q->term_isig = nullptr;
     if (mlp) {
       alloc_term(q->term_arena, q, q->diff_tb);
       di.term_p = q->diff_tb.P;
@@ -2247,6 +2252,13 @@ heomgb_status heomgb_qme_set_terminator(heomgb_qme* q, heomgb_mlp* mlp) {
       }
       q->term_cke = q->term_arena.upload(to_f2(cke), q->stream());
       q->term_sgn = q->term_arena.upload(sgn, q->stream());
+      float2* rowf = static_cast<float2*>(
+          q->term_arena.alloc(sizeof(float2) * std::max<size_t>(1, static_cast<size_t>(q->diff_tb.n_tier) * K)));
+      float2* isig = static_cast<float2*>(q->term_arena.alloc(sizeof(float2) * std::max(1, K)));
+      ck(launch_term_tables(term_model(q), q->diff_tb.first, q->diff_tb.n_tier, rowf, isig, q->stream()),
+         "terminator tables");
+      q->term_rowf = rowf;
+      q->term_isig = isig;
       ck(cudaStreamSynchronize(q->stream()), "terminator tables");
     }
     build_plan(q->diff_plan, {di}, q->diff_plan.block, q->diff_plan.ept, q->diff_plan.min_blocks,

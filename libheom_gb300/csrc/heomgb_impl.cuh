@@ -353,17 +353,61 @@ struct TermModel {
   // head's sign(Re(v_a - v_b)), for V of mode k's bath
   const float2* cke = nullptr;    // K * n2
   const float* sgn = nullptr;     // K * n2
+  const float2* rowf = nullptr;   // n_tier * K: (n_k + 1) / (ngamma_l + gamma_kk) of the tier-N ADOs
+  const float2* isig = nullptr;   // K: 1 / sigma_k
 };
+cudaError_t launch_term_tables(const TermModel& tm, int first, int n_tier, float2* rowf, float2* isig, cudaStream_t s);
 cudaError_t term_enqueue(heomgb_mlp* M, const TermBuffers& tb, const TermModel& tm, const TermInput& in,
                          bool y_float, cudaStream_t s);
-// The fused inference (tcgemm.cu): features, three tensor-core layers and the
+// Where a weight goes when it changes: the plain BF16 copy (parameter order)
+// and, for sizes that the fused closure kernels take, the packed operands
+// (tcore.cuh): f[l] of layer l (rows: outputs, k: inputs), t[0] / t[1] the
+// transposes of layers 2 and 3 (rows: inputs, k: outputs).
+struct WeightStore {
+  __nv_bfloat16* wb = nullptr;
+  __nv_bfloat16* f[3] = {nullptr, nullptr, nullptr};  // f[0] null: no packed copies
+  __nv_bfloat16* t[2] = {nullptr, nullptr};
+  long long off[6] = {0, 0, 0, 0, 0, 0};
+  int din = 0, h = 0, dout = 0;
+};
+// One training pass (closure.cu): forward, loss, backward and the gradients.
+struct TrainArgs {
+  const float* X;              // B x din
+  const float* T;              // B x (5 n2 or dout)
+  int B, din, h, dout, kind, n2;
+  const float *b1, *b2, *b3;
+  const __nv_bfloat16 *W1, *W2, *W3, *W3t, *W2t;  // packed
+  unsigned char* img;          // train_image_bytes: the operands of the weight gradients
+  float* g;                    // the gradient (parameter order)
+  long long off[6];
+  float* loss;                 // train_tiles: the tiles' losses
+  int* err;                    // set to 1 if a tensor-core or copy wait ran out
+};
+struct AdamArgs {
+  long long n_params;
+  const float* g;
+  float *w, *m, *v;
+  WeightStore wt;
+  float lr, b1, b2, eps, c1, c2;
+  const int* err;
+};
+bool train_fused_ok(int din, int h, int dout, int kind, int n2);
+bool closure_sizes_ok(int din, int h, int dout);
+size_t closure_pack_elems(int which, int din, int h, int dout);  // f[0], f[1], f[2], t[0], t[1]
+int train_tiles(int batch);
+size_t train_image_bytes(int din, int h, int dout, int tiles);
+cudaError_t launch_train(const TrainArgs& a, cudaStream_t s);
+cudaError_t launch_adam(const AdamArgs& a, cudaStream_t s);
+cudaError_t launch_weights(const float* w, const WeightStore& wt, long long n, cudaStream_t s);
+// The fused inference (closure.cu): features, three tensor-core layers and the
 // gain head of the terminator in one launch.
 struct TermMlpArgs {
   TermInput in;
   TermModel tm;
-  int first, n_tier, apt;      // tier-N ADOs [first, first + n_tier); ADOs per CTA (apt K <= 128)
+  int first, n_tier;           // tier-N ADOs [first, first + n_tier)
+  int apt;                     // ADOs per CTA (set by the launcher)
   int din, h, dout;
-  const __nv_bfloat16* W1;
+  const __nv_bfloat16* W1;     // packed
   const __nv_bfloat16* W2;
   const __nv_bfloat16* W3;
   const float* b1;
@@ -372,8 +416,8 @@ struct TermMlpArgs {
   float2* P;                   // n_tier K rows of n2 predictions
   int* err;                    // set to 1 if a tensor-core wait ran out
 };
-bool term_fused_ok(int din, int h, int dout, int K);
-cudaError_t launch_term_fused(const TermMlpArgs& a, bool y_float, cudaStream_t s);
+bool term_fused_ok(int din, int h, int dout, int K, int n2);
+cudaError_t launch_term_fused(TermMlpArgs a, int n_sm, bool y_float, cudaStream_t s);
 void mlp_dims(const heomgb_mlp* M, int* din, int* h, int* dout);
 // true (and the flag cleared) if a tensor-core GEMM of M's inference gave up a wait
 bool mlp_take_error(heomgb_mlp* M, cudaStream_t s);

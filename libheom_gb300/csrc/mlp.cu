@@ -116,29 +116,6 @@ __global__ void k_gain_loss(const float* __restrict__ Y, const float* __restrict
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// Adam on the FP32 masters, then refresh the BF16 copies.
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       __nv_bfloat16* __restrict__ wb, long long n, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    wb[i] = __float2bfloat16(wi);
-  }
-}
-
-__global__ void k_to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__ wb, long long n) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    wb[i] = __float2bfloat16(w[i]);
-}
-
 void ckm(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -163,7 +140,14 @@ struct heomgb_mlp {
   int cap = 0;                  // batch capacity of the activation buffers
   float *a1 = nullptr, *p1 = nullptr, *a2 = nullptr, *p2 = nullptr, *y = nullptr, *d = nullptr, *d2 = nullptr;
   float* part = nullptr;
-  int* err = nullptr;           // set by a tensor-core GEMM whose wait ran out
+  int* err = nullptr;           // set by a tensor-core kernel whose wait ran out
+  int* tstat = nullptr;         // status of the fused training pass, and its pinned mirror
+  int* status = nullptr;
+  WeightStore wt;               // every BF16 copy of the weights
+  __nv_bfloat16* packs = nullptr;
+  int n_sm = 0;
+  int tiles = 0;                // capacity of the fused training pass
+  unsigned char* timg = nullptr;
   cudaStream_t s = nullptr;
   void free_acts() {
     for (float* p : {a1, p1, a2, p2, y, d, d2, part}) cudaFree(p);
@@ -184,8 +168,28 @@ struct heomgb_mlp {
     ckm(cudaMalloc(&part, sizeof(float) * 1024), "mlp alloc");
     cap = B;
   }
+  // buffers of the fused training pass, and its status: the error flag, then the tiles' losses
+  void ensure_train(int t) {
+    if (t <= tiles) return;
+    tiles = 0;
+    cudaFree(timg);
+    cudaFree(tstat);
+    timg = nullptr;
+    tstat = nullptr;
+    if (status) cudaFreeHost(status);
+    status = nullptr;
+    ckm(cudaMalloc(&timg, train_image_bytes(din, h, dout, t)), "mlp alloc");
+    ckm(cudaMalloc(&tstat, sizeof(int) * (1 + static_cast<size_t>(t))), "mlp alloc");
+    ckm(cudaMemsetAsync(tstat, 0, sizeof(int), s), "memset");
+    ckm(cudaMallocHost(&status, sizeof(int) * (1 + static_cast<size_t>(t))), "mlp alloc");
+    tiles = t;
+  }
   ~heomgb_mlp() {
     free_acts();
+    cudaFree(timg);
+    cudaFree(tstat);
+    cudaFree(packs);
+    if (status) cudaFreeHost(status);
     for (void* p : {static_cast<void*>(w), static_cast<void*>(wb), static_cast<void*>(g), static_cast<void*>(m),
                     static_cast<void*>(v), static_cast<void*>(err)})
       cudaFree(p);
@@ -268,6 +272,72 @@ void data_grad(heomgb_mlp* M, const float* dZ, int layer, const float* PRE, floa
   const int din = layer == 0 ? M->din : M->h, dout = layer == 2 ? M->dout : M->h;
   gemm(M, op_f32(dZ, dout, 1), op_bf16(M->wb + M->off[2 * layer], 1, din), dH, din, nullptr,
        const_cast<float*>(PRE), B, din, dout, GEMM_GELU_GRAD, M->s);
+}
+
+// One Adam step from the gradient in M->g (queued after it), unless *err is set.
+void adam(heomgb_mlp* M, float lr, const int* err) {
+  AdamArgs a{};
+  a.n_params = M->n_params;
+  a.g = M->g;
+  a.w = M->w;
+  a.m = M->m;
+  a.v = M->v;
+  a.wt = M->wt;
+  a.err = err;
+  a.lr = lr;
+  a.b1 = 0.9f;
+  a.b2 = 0.999f;
+  a.eps = 1e-8f;
+  a.c1 = 1.f - std::pow(a.b1, static_cast<float>(M->step + 1));
+  a.c2 = 1.f - std::pow(a.b2, static_cast<float>(M->step + 1));
+  ckm(launch_adam(a, M->s), "adam");
+}
+
+// Sizes that the fused training pass takes (k_train, k_dw: forward, loss,
+// backward and weight gradients in two launches); others run the GEMMs one by one.
+bool fused(const heomgb_mlp* M) {
+  return M->wt.f[0] && train_fused_ok(M->din, M->h, M->dout, M->loss_kind, M->loss_n2);
+}
+
+// The fused pass: the gradient to M->g, then (step) an Adam step; returns the loss.
+float train_pass(heomgb_mlp* M, const float* X, const float* T, int B, float lr, bool step) {
+  const int tiles = train_tiles(B);
+  M->ensure_train(tiles);
+  TrainArgs a{};
+  a.X = X;
+  a.T = T;
+  a.B = B;
+  a.din = M->din;
+  a.h = M->h;
+  a.dout = M->dout;
+  a.kind = M->loss_kind;
+  a.n2 = M->loss_n2;
+  a.b1 = M->w + M->off[1];
+  a.b2 = M->w + M->off[3];
+  a.b3 = M->w + M->off[5];
+  a.W1 = M->wt.f[0];
+  a.W2 = M->wt.f[1];
+  a.W3 = M->wt.f[2];
+  a.W2t = M->wt.t[0];
+  a.W3t = M->wt.t[1];
+  a.img = M->timg;
+  a.g = M->g;
+  for (int i = 0; i < 6; ++i) a.off[i] = M->off[i];
+  a.loss = reinterpret_cast<float*>(M->tstat + 1);
+  a.err = M->tstat;
+  ckm(launch_train(a, M->s), "mlp training pass");
+  if (step) adam(M, lr, M->tstat);
+  ckm(cudaMemcpyAsync(M->status, M->tstat, sizeof(int) * (1 + static_cast<size_t>(tiles)), cudaMemcpyDeviceToHost,
+                      M->s),
+      "mlp status");
+  ckm(cudaStreamSynchronize(M->s), "mlp sync");
+  if (M->status[0]) {
+    ckm(cudaMemsetAsync(M->tstat, 0, sizeof(int), M->s), "mlp status reset");
+    throw std::runtime_error("tensor-core GEMM did not complete (a bounded wait ran out)");
+  }
+  double loss = 0;
+  for (int i = 0; i < tiles; ++i) loss += reinterpret_cast<const float*>(M->status)[1 + i];
+  return static_cast<float>(loss / (M->loss_kind == 1 ? static_cast<double>(B) : static_cast<double>(B) * M->dout));
 }
 
 // Forward + backward: fills M->g with the gradient of the loss; returns the loss.
@@ -417,25 +487,24 @@ cudaError_t term_enqueue(heomgb_mlp* M, const TermBuffers& tb, const TermModel& 
   // one fused launch (features, three tensor-core layers, gain head) where the
   // sizes allow it; HEOMGB_TERM_FUSED=0 keeps the five-launch form below
   const char* fused_env = std::getenv("HEOMGB_TERM_FUSED");
-  if (term_fused_ok(M->din, M->h, M->dout, tb.K) && !(fused_env && std::string(fused_env) == "0")) {
+  if (M->wt.f[0] && term_fused_ok(M->din, M->h, M->dout, tb.K, tb.n2) && !(fused_env && std::string(fused_env) == "0")) {
     TermMlpArgs a{};
     a.in = in;
     a.tm = tm;
     a.first = tb.first;
     a.n_tier = tb.n_tier;
-    a.apt = 128 / tb.K;
     a.din = M->din;
     a.h = M->h;
     a.dout = M->dout;
-    a.W1 = M->wb + M->off[0];
-    a.W2 = M->wb + M->off[2];
-    a.W3 = M->wb + M->off[4];
+    a.W1 = M->wt.f[0];
+    a.W2 = M->wt.f[1];
+    a.W3 = M->wt.f[2];
     a.b1 = M->w + M->off[1];
     a.b2 = M->w + M->off[3];
     a.b3 = M->w + M->off[5];
     a.P = tb.P;
     a.err = M->err;
-    return launch_term_fused(a, y_float, s);
+    return launch_term_fused(a, M->n_sm, y_float, s);
   }
   const int R = tb.n_tier * tb.K;
   if (y_float)
@@ -508,14 +577,32 @@ heomgb_status heomgb_mlp_create(int d_in, int d_hidden, int d_out, unsigned long
     ckm(cudaMalloc(&M->m, fb), "mlp alloc");
     ckm(cudaMalloc(&M->v, fb), "mlp alloc");
     ckm(cudaMalloc(&M->wb, sizeof(__nv_bfloat16) * o), "mlp alloc");
+    int dev = 0;
+    ckm(cudaGetDevice(&dev), "device");
+    ckm(cudaDeviceGetAttribute(&M->n_sm, cudaDevAttrMultiProcessorCount, dev), "device attribute");
     ckm(cudaMalloc(&M->err, sizeof(int)), "mlp alloc");
     ckm(cudaMemsetAsync(M->err, 0, sizeof(int), M->s), "memset");
+    M->wt.wb = M->wb;
+    for (int i = 0; i < 6; ++i) M->wt.off[i] = M->off[i];
+    M->wt.din = d_in;
+    M->wt.h = d_hidden;
+    M->wt.dout = d_out;
+    if (closure_sizes_ok(d_in, d_hidden, d_out)) {  // the packed operands, zero where padded
+      size_t total = 0;
+      for (int i = 0; i < 5; ++i) total += closure_pack_elems(i, d_in, d_hidden, d_out);
+      ckm(cudaMalloc(&M->packs, sizeof(__nv_bfloat16) * total), "mlp alloc");
+      ckm(cudaMemsetAsync(M->packs, 0, sizeof(__nv_bfloat16) * total, M->s), "memset");
+      __nv_bfloat16* p = M->packs;
+      for (int i = 0; i < 5; ++i) {
+        (i < 3 ? M->wt.f[i] : M->wt.t[i - 3]) = p;
+        p += closure_pack_elems(i, d_in, d_hidden, d_out);
+      }
+    }
     ckm(cudaMemcpyAsync(M->w, w.data(), fb, cudaMemcpyHostToDevice, M->s), "mlp init");
     ckm(cudaMemsetAsync(M->g, 0, fb, M->s), "memset");
     ckm(cudaMemsetAsync(M->m, 0, fb, M->s), "memset");
     ckm(cudaMemsetAsync(M->v, 0, fb, M->s), "memset");
-    k_to_bf16<<<grid_for(o), 256, 0, M->s>>>(M->w, M->wb, o);
-    ++g_launches;
+    ckm(launch_weights(M->w, M->wt, o, M->s), "mlp weights");
     ckm(cudaStreamSynchronize(M->s), "mlp init sync");
     *out = M.release();
   });
@@ -551,8 +638,7 @@ heomgb_status heomgb_mlp_set_params(heomgb_mlp* M, const float* params) {
   return mguard([&] {
     if (!M || !params) throw std::invalid_argument("null argument");
     ckm(cudaMemcpyAsync(M->w, params, sizeof(float) * M->n_params, cudaMemcpyHostToDevice, M->s), "copy");
-    k_to_bf16<<<grid_for(M->n_params), 256, 0, M->s>>>(M->w, M->wb, M->n_params);
-    ++g_launches;
+    ckm(launch_weights(M->w, M->wt, M->n_params, M->s), "mlp weights");
     ckm(cudaStreamSynchronize(M->s), "sync");
   });
 }
@@ -579,7 +665,7 @@ heomgb_status heomgb_mlp_gradients(heomgb_mlp* M, const float* x_dev, const floa
                                    float* grad_host, float* loss) {
   return mguard([&] {
     if (!M || !x_dev || !t_dev || batch < 1) throw std::invalid_argument("bad argument");
-    const float l = backward(M, x_dev, t_dev, batch);
+    const float l = fused(M) ? train_pass(M, x_dev, t_dev, batch, 0.f, false) : backward(M, x_dev, t_dev, batch);
     if (loss) *loss = l;
     if (grad_host) {
       ckm(cudaMemcpyAsync(grad_host, M->g, sizeof(float) * M->n_params, cudaMemcpyDeviceToHost, M->s), "copy");
@@ -592,16 +678,15 @@ heomgb_status heomgb_mlp_train_step(heomgb_mlp* M, const float* x_dev, const flo
                                     float* loss) {
   return mguard([&] {
     if (!M || !x_dev || !t_dev || batch < 1) throw std::invalid_argument("bad argument");
-    const float l = backward(M, x_dev, t_dev, batch);
+    float l;
+    if (fused(M)) {
+      l = train_pass(M, x_dev, t_dev, batch, lr, true);
+    } else {
+      l = backward(M, x_dev, t_dev, batch);
+      adam(M, lr, M->err);
+      ckm(cudaStreamSynchronize(M->s), "sync");
+    }
     M->step += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - std::pow(b1, static_cast<float>(M->step));
-    const float c2 = 1.f - std::pow(b2, static_cast<float>(M->step));
-    k_adam<<<grid_for(M->n_params), 256, 0, M->s>>>(M->w, M->g, M->m, M->v, M->wb, M->n_params, lr, b1, b2, 1e-8f,
-                                                    c1, c2);
-    ++g_launches;
-    ckm(cudaGetLastError(), "adam");
-    ckm(cudaStreamSynchronize(M->s), "sync");
     if (loss) *loss = l;
   });
 }

@@ -225,6 +225,11 @@ heomgb_status heomgb_qme_solver_site_kernel(const heomgb_qme_solver* qs, int* on
  * (rk4.h:40-65) and lsrk4::solve_fixed_step (lsrk4.h:32-47) issue every
  * stage's BLAS calls from the host. */
 heomgb_status heomgb_qme_solver_resident(const heomgb_qme_solver* qs, int* on, int* grid, int* ados_per_cta);
+/* Whether fixed steps run as cluster-resident intervals (one launch per output
+ * interval, a thread-block cluster of `size` CTAs of `block` threads per bin of
+ * instances).  No reference counterpart. */
+heomgb_status heomgb_qme_solver_cluster(const heomgb_qme_solver* qs, int* on, int* size, int* clusters, int* block);
+
 /* 1 when the solver runs each fixed-step (rk4, lsrk4) output interval as one launch of
  * instance-resident bins (diagonal-coupling path, every instance inside one
  * CTA: its stage inputs in shared memory, no grid-wide synchronisation), else

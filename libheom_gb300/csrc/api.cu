@@ -413,6 +413,14 @@ struct heomgb_qme_solver {
   DeviceArena loc_arena;
   const int* loc_bin_ptr = nullptr;
   const int* loc_bin_inst = nullptr;
+  // cluster-resident fixed-step intervals (k_cluster): one launch per output
+  // interval, a thread-block cluster per bin of instances
+  bool cluster = false;
+  int clu_size = 0, clu_bins = 0, clu_block = 0, clu_ept = 0;
+  size_t clu_smem = 0;
+  DeviceArena clu_arena;
+  ClusterArgs clu{};
+  float loc_step_ms = 0.f;  // the instance-resident plan's time per step (0: not timed)
   float stage_ms = 0.f;     // the autotuned stage kernel's time per launch (0: not timed)
   float res_step_ms = 0.f;  // the resident fixed-step plan's time per step (0: not timed)
   // batch solvers run on a stream of their own (sub-batches of one batch run
@@ -812,8 +820,11 @@ void build_model(heomgb_qme* q) {
         pp[e + 1] = static_cast<int>(pmode.size());
         pm[e + 1] = static_cast<int>(mmode.size());
       }
-    int max_terms = 0;
-    for (int e = 0; e < n2; ++e) max_terms = std::max({max_terms, pp[e + 1] - pp[e], pm[e + 1] - pm[e]});
+    int max_terms = 0, sum_terms = 0;
+    for (int e = 0; e < n2; ++e) {
+      max_terms = std::max({max_terms, pp[e + 1] - pp[e], pm[e + 1] - pm[e]});
+      sum_terms = std::max(sum_terms, pp[e + 1] - pp[e] + pm[e + 1] - pm[e]);
+    }
     m.plus_ptr = q->arena.upload(pp, s);
     m.plus_mode = q->arena.upload(pmode, s);
     m.minus_ptr = q->arena.upload(pm, s);
@@ -839,6 +850,14 @@ void build_model(heomgb_qme* q) {
     }
     di.sqrt_norm = m.sqrt_norm;
     di.max_terms = max_terms;
+    di.sum_terms = sum_terms;
+    {
+      std::vector<int> eo(n2);
+      for (int e = 0; e < n2; ++e) eo[e] = e;
+      std::stable_sort(eo.begin(), eo.end(),
+                       [&](int x, int y) { return pp[x + 1] - pp[x] + pm[x + 1] - pm[x] > pp[y + 1] - pp[y] + pm[y + 1] - pm[y]; });
+      di.e_order = q->arena.upload(eo, s);
+    }
     di.elem_off = 0;
     di.p1 = m.p1;
     di.m1 = m.m1;
@@ -1092,6 +1111,7 @@ void run_diff_rm(heomgb_qme* q, double2* drho, const double2* rho, const double*
 void autotune(heomgb_qme_solver* qs);
 void plan_resident(heomgb_qme_solver* qs);
 void plan_local(heomgb_qme_solver* qs);
+void plan_cluster(heomgb_qme_solver* qs);
 
 // The resident kernel of the solver's scheme.
 int resident_scheme(const heomgb_qme_solver* qs) {
@@ -1184,6 +1204,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
   qs->partials = static_cast<double*>(A.alloc(sizeof(double) * std::max(qs->grid, 1)));
   plan_resident(qs);
   plan_local(qs);
+  plan_cluster(qs);
 }
 
 // Tile shape search for the diagonal-coupling kernel: CTA size x elements per
@@ -1646,10 +1667,177 @@ void plan_local(heomgb_qme_solver* qs) {
   qs->loc_bin_ptr = qs->loc_arena.upload(sh.ptr, qs->stream);
   qs->loc_bin_inst = qs->loc_arena.upload(sh.list, qs->stream);
   ck(cudaStreamSynchronize(qs->stream), "local plan upload");
+  qs->loc_step_ms = best_ms / 4.f;
   qs->loc_grid = sh.grid;
   qs->loc_block = sh.block;
   qs->loc_smem = sh.smem;
   qs->local = true;
+}
+
+// Cluster-resident fixed steps (k_cluster) apply to RK4 and LSRK4 on the
+// diagonal-coupling path without a terminator when the bins fit the clusters'
+// shared memory.  For every cluster size, as many bins as clusters are resident
+// at once (at most one per instance), the instances packed largest
+// first into the least-loaded bin; every size runs a few steps over the
+// solver's zeroed buffers.  The fastest
+// replaces whatever plan the solver has (timed the same way) where it is
+// faster: small models and batches whose stages are latency, not work (FP64
+// spin-boson depth 10: 3.2 us a stage in the cooperative interval, 2.0 here;
+// the 7-site depth-3 hierarchy: 1.9 and 4, so it keeps the other).
+// HEOMGB_CLUSTER=0 keeps it out, =1 takes it without the comparison; a plan
+// pinned by HEOMGB_TILE, HEOMGB_RESIDENT or HEOMGB_LOCAL stays.
+void plan_cluster(heomgb_qme_solver* qs) {
+  const NvtxRange range("heomgb plan: cluster-resident bins");
+  heomgb_qme* q = qs->q;
+  qs->cluster = false;
+  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || q->path != PATH_DIAG || qs->term) return;
+  bool force = false;
+  if (const char* env = std::getenv("HEOMGB_CLUSTER")) {
+    if (std::string(env) == "0") return;
+    force = std::string(env) == "1";
+  }
+  for (const char* pin : {"HEOMGB_TILE", "HEOMGB_RESIDENT", "HEOMGB_LOCAL", "HEOMGB_RESIDENT_PER_SM", "HEOMGB_RESIDENT_EPT"})
+    if (std::getenv(pin) && !force) return;
+  int pin_size = 0;
+  if (const char* env = std::getenv("HEOMGB_CLUSTER_SIZE")) pin_size = std::atoi(env);
+  const std::vector<DiagInst>& insts = qs->plan.inst;
+  const bool mixed = qs->mixed;
+  const int scheme = resident_scheme(qs);
+  int terms = 1;
+  for (const DiagInst& I : insts) {
+    if (I.term_p || I.n > 64) return;
+    terms = std::max(terms, I.sum_terms);
+  }
+  std::vector<int> order(insts.size());
+  for (size_t i = 0; i < order.size(); ++i) order[i] = static_cast<int>(i);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    return static_cast<long long>(insts[x].n2) * insts[x].nh > static_cast<long long>(insts[y].n2) * insts[y].nh;
+  });
+  struct Shape {
+    int size, bins, block, ept, ecap;
+    size_t smem;
+    std::vector<int> ptr, list;
+  };
+  std::vector<Shape> shapes;
+  for (int size = 1; size <= kClusterMaxSize; size *= 2) {
+    if (pin_size && size != pin_size) continue;
+    // clusters resident at once (a cluster's CTAs share a GPC, so not every SM gets one)
+    const int active = cluster_active(mixed, scheme, 1, size, kClusterMaxBlock, 200 * 1024);
+    if (active < 1) continue;
+    const int want = static_cast<int>(std::min<size_t>(insts.size(), static_cast<size_t>(active)));
+    std::vector<long long> load(want, 0);
+    std::vector<std::vector<int>> bins(want);
+    bool fits = true;
+    for (int i : order) {
+      int pick_b = -1;
+      for (int b = 0; b < want; ++b)
+        if (static_cast<int>(bins[b].size()) < kClusterMaxInst && (pick_b < 0 || load[b] < load[pick_b])) pick_b = b;
+      if (pick_b < 0) {
+        fits = false;
+        break;
+      }
+      bins[pick_b].push_back(i);
+      load[pick_b] += static_cast<long long>(insts[i].n2) * insts[i].nh;
+    }
+    if (!fits) continue;
+    Shape sh{};
+    sh.size = size;
+    sh.bins = want;
+    sh.ptr.push_back(0);
+    int h_max = 0;
+    long long most = 0;
+    for (const std::vector<int>& b : bins) {
+      std::vector<int> n2, nh;
+      int h = 0;
+      for (int i : b) {
+        n2.push_back(insts[i].n2);
+        nh.push_back(insts[i].nh);
+        h += insts[i].n2;
+        sh.list.push_back(i);
+      }
+      sh.ptr.push_back(static_cast<int>(sh.list.size()));
+      h_max = std::max(h_max, h);
+      long long total = 0;
+      for (size_t i = 0; i < n2.size(); ++i) total += static_cast<long long>(n2[i]) * nh[i];
+      if (total > (1LL << 20)) {
+        fits = false;
+        break;
+      }
+      most = std::max<long long>(most, cluster_elements(n2.data(), nh.data(), static_cast<int>(n2.size()), size));
+    }
+    if (!fits) continue;
+    sh.ecap = static_cast<int>((most + 1) / 2 * 2);
+    sh.smem = cluster_smem(h_max, sh.ecap, terms, mixed);
+    if (sh.smem > 200 * 1024) continue;
+    const int lanes = sh.ecap * cluster_lanes(mixed);
+    for (int ept : {1, 2, 4}) {  // the fewest elements per thread that the block size allows
+      sh.ept = ept;
+      sh.block = std::max(32, ((lanes + ept - 1) / ept + 31) / 32 * 32);
+      if (sh.block > (ept > 2 ? 512 : kClusterMaxBlock)) continue;
+      if (cluster_active(mixed, scheme, ept, size, sh.block, sh.smem) >= 1) shapes.push_back(sh);
+      break;
+    }
+  }
+  if (shapes.empty()) return;
+  ck(cudaMemsetAsync(qs->S[0], 0, sizeof(double2) * qs->N, qs->stream), "memset");
+  cudaEvent_t e0, e1;
+  ck(cudaEventCreate(&e0), "event");
+  ck(cudaEventCreate(&e1), "event");
+  const bool tune_log = std::getenv("HEOMGB_TUNE_LOG") && std::string(std::getenv("HEOMGB_TUNE_LOG")) == "1";
+  float best_ms = 1e30f;
+  size_t best = 0;
+  // the interval's set-up (the bath-term tables) is paid once, so a step's time
+  // is the difference of a long and a short interval
+  DeviceArena tab;
+  for (size_t i = 0; i < shapes.size(); ++i) {
+    const Shape& sh = shapes[i];
+    ClusterArgs a{};
+    a.inst = qs->plan.ds.inst;
+    a.bin_ptr = tab.upload(sh.ptr, qs->stream);
+    a.bin_inst = tab.upload(sh.list, qs->stream);
+    a.S = qs->S[0];
+    a.dt_step = a.dt_last = 1e-3;
+    a.ecap = sh.ecap;
+    a.terms = terms;
+    float t[2] = {1e30f, 1e30f};
+    for (int r = 0; r < 4; ++r) {  // best of two
+      a.n_steps = (r & 1) ? 11 : 3;
+      ck(cudaEventRecord(e0, qs->stream), "event");
+      ck(launch_cluster(a, mixed, scheme, sh.ept, sh.size, sh.bins, sh.block, sh.smem, qs->stream), "cluster tune");
+      ck(cudaEventRecord(e1, qs->stream), "event");
+      ck(cudaEventSynchronize(e1), "event sync");
+      float ms = 0.f;
+      ck(cudaEventElapsedTime(&ms, e0, e1), "event time");
+      t[r & 1] = std::min(t[r & 1], ms);
+    }
+    const float ms = std::max(t[1] - t[0], 0.1f * t[1]) / 8.f;
+    if (tune_log)
+      std::fprintf(stderr, "heomgb tune: cluster %d bins %d block %d ept %d: %.4f ms per step\n", sh.size, sh.bins,
+                   sh.block, sh.ept, ms);
+    if (ms < best_ms) {
+      best_ms = ms;
+      best = i;
+    }
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  const float rival = qs->local ? qs->loc_step_ms : qs->resident ? qs->res_step_ms : 4.f * qs->stage_ms;
+  if (!force && !(best_ms < rival)) return;
+  const Shape& sh = shapes[best];
+  qs->clu.inst = qs->plan.ds.inst;
+  qs->clu.bin_ptr = qs->clu_arena.upload(sh.ptr, qs->stream);
+  qs->clu.bin_inst = qs->clu_arena.upload(sh.list, qs->stream);
+  ck(cudaStreamSynchronize(qs->stream), "cluster plan upload");
+  qs->clu.S = qs->S[0];
+  qs->clu.ecap = sh.ecap;
+  qs->clu.terms = terms;
+  qs->clu_size = sh.size;
+  qs->clu_bins = sh.bins;
+  qs->clu_block = sh.block;
+  qs->clu_ept = sh.ept;
+  qs->clu_smem = sh.smem;
+  qs->cluster = true;
+  qs->local = qs->resident = false;
 }
 
 Stage solver_stage(heomgb_qme_solver* qs) {
@@ -1814,6 +2002,22 @@ void solve_fixed(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwarg
     }
     t += d;
     if (++m > cap) throw numeric_error("fixed-step loop does not terminate");
+  }
+  if (qs->cluster) {  // the whole interval as one launch of clusters (k_cluster)
+    ClusterArgs a = qs->clu;
+    a.n_steps = m;
+    a.dt_step = dt;
+    a.dt_last = last;
+    busy_begin(qs);
+    ck(launch_cluster(a, qs->mixed, resident_scheme(qs), qs->clu_ept, qs->clu_size, qs->clu_bins, qs->clu_block,
+                      qs->clu_smem, qs->stream),
+       "cluster-resident interval");
+    busy_end(qs);
+    qs->replayed_kernels += 1;
+    qs->n_rhs += 4 * (m + 1);
+    qs->n_attempts += m + 1;
+    qs->n_accepted += m + 1;
+    return;
   }
   if (qs->local) {  // the whole interval as one launch of instance-resident bins (k_fixed_local)
     LocalArgs a{};
@@ -2005,7 +2209,7 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
     } else {
       ck(cudaMemcpyAsync(qs->S[0], rho, bytes, in_kind, qs->stream), "state in");
     }
-    state_to_bulk(qs, 0);
+    if (!qs->cluster) state_to_bulk(qs, 0);  // k_cluster forms the FP32 copy itself
     int cur = 0;
     if (qs->kind == HEOMGB_RKDP)
       cur = qs->resident ? solve_resident(qs, t_list[i], t_list[i + 1], kw, 0)
@@ -2436,6 +2640,16 @@ heomgb_status heomgb_qme_solver_resident(const heomgb_qme_solver* qs, int* on, i
     *on = qs->resident ? 1 : 0;
     if (grid) *grid = qs->resident ? qs->res_grid : 0;
     if (ados_per_cta) *ados_per_cta = qs->resident ? qs->res_apc : 0;
+  });
+}
+
+heomgb_status heomgb_qme_solver_cluster(const heomgb_qme_solver* qs, int* on, int* size, int* clusters, int* block) {
+  return guard([&] {
+    require(qs != nullptr, "null qme_solver");
+    if (on) *on = qs->cluster ? 1 : 0;
+    if (size) *size = qs->clu_size;
+    if (clusters) *clusters = qs->clu_bins;
+    if (block) *block = qs->clu_block;
   });
 }
 

@@ -150,6 +150,8 @@ struct DiagInst {
   int sqrt_norm;            // 1: +1 terms scale by sqrt(n_k+1), -1 terms by sqrt(n_k) (else 1 and n_k)
   int h_sym;                // H real and symmetric (the tensor-core commutator's condition)
   int max_terms;            // max over elements of max(+1 terms, -1 terms)
+  int sum_terms;            // max over elements of (+1 terms) + (-1 terms)
+  const int* e_order;       // n2: the elements, those with the most terms first
   const int* plus_any;      // per ADO: 1 if any ptr_p1 entry is a real ADO (0 on the deepest tier)
   // FP64 coefficients scaled by the occupation n_k = 0..max_depth (row p*(max_depth+1) + n_k):
   // -1 terms n_k c_minus[p] (sqrt(n_k) c_minus[p] under sqrt normalisation); +1 terms
@@ -255,6 +257,29 @@ size_t local_bin_smem(const int* n2, const int* nh, int count, bool mixed);
 int local_blocks_per_sm(bool mixed, int scheme, int block, size_t smem);
 cudaError_t launch_local(const LocalArgs& args, bool mixed, int scheme, int grid, int block, size_t smem,
                          cudaStream_t s);
+
+// Cluster-resident fixed-step intervals (cluster.cu): a thread-block cluster
+// of `size` CTAs per bin of whole instances.  The scheme is kResidentRk4 or
+// kResidentLs.
+constexpr int kClusterMaxInst = 32;  // instances per bin
+constexpr int kClusterMaxSize = 16;  // CTAs per cluster
+constexpr int kClusterMaxBlock = 448;  // threads per CTA (512 with four elements per thread)
+struct ClusterArgs {
+  const DiagInst* inst;     // device array of the instances
+  const int* bin_ptr;       // bin b holds instances bin_inst[bin_ptr[b] .. bin_ptr[b+1])
+  const int* bin_inst;
+  double2* S;               // FP64 state (updated in place)
+  long long n_steps;        // steps of dt_step before the last step of dt_last
+  double dt_step, dt_last;
+  int ecap;                 // elements of the fullest CTA
+  int terms;                // bath-term slots per element
+};
+int cluster_lanes(bool mixed);  // lanes per element
+int cluster_elements(const int* n2, const int* nh, int count, int size);  // of a bin's fullest CTA
+size_t cluster_smem(int h_elems, int ecap, int terms, bool mixed);
+int cluster_active(bool mixed, int scheme, int ept, int size, int block, size_t smem);
+cudaError_t launch_cluster(const ClusterArgs& args, bool mixed, int scheme, int ept, int size, int bins, int block,
+                           size_t smem, cudaStream_t s);
 
 // Launchers (kernels.cu).  `mixed` selects FP32 bulk arithmetic; `in_double`
 // says the RHS input is a double2 array even in mixed mode.  `ds` describes

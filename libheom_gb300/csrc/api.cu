@@ -2197,23 +2197,28 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
   const size_t bytes = sizeof(double2) * qs->N;
   const cudaMemcpyKind in_kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   const cudaMemcpyKind out_kind = host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-  // solver_base::solve (solver_base.h:64-79)
+  // solver_base::solve (solver_base.h:64-79).  Without a callback nobody sees or
+  // changes rho between two intervals, so only the first reads it; every
+  // interval still writes it back, so a failed one leaves the last good state.
+  int cur = 0;
   for (int i = 0; i < n_t - 1; ++i) {
     if (cb) {
       if (!host) ck(cudaStreamSynchronize(qs->stream), "sync before callback");
       cb(t_list[i], user);
     }
-    if (qs->col_major) {  // the caller's ADOs are column-major: transpose at the boundary
-      ck(cudaMemcpyAsync(qs->otmp, rho, bytes, in_kind, qs->stream), "state in");
-      transpose_instances(qs, qs->otmp, qs->S[0]);
-    } else {
-      ck(cudaMemcpyAsync(qs->S[0], rho, bytes, in_kind, qs->stream), "state in");
+    if (i == 0 || cb) {
+      if (qs->col_major) {  // the caller's ADOs are column-major: transpose at the boundary
+        ck(cudaMemcpyAsync(qs->otmp, rho, bytes, in_kind, qs->stream), "state in");
+        transpose_instances(qs, qs->otmp, qs->S[0]);
+      } else {
+        ck(cudaMemcpyAsync(qs->S[0], rho, bytes, in_kind, qs->stream), "state in");
+      }
+      if (!qs->cluster) state_to_bulk(qs, 0);  // k_cluster forms the FP32 copy itself
+      cur = 0;
     }
-    if (!qs->cluster) state_to_bulk(qs, 0);  // k_cluster forms the FP32 copy itself
-    int cur = 0;
     if (qs->kind == HEOMGB_RKDP)
-      cur = qs->resident ? solve_resident(qs, t_list[i], t_list[i + 1], kw, 0)
-                         : solve_adaptive(qs, t_list[i], t_list[i + 1], kw, 0);
+      cur = qs->resident ? solve_resident(qs, t_list[i], t_list[i + 1], kw, cur)
+                         : solve_adaptive(qs, t_list[i], t_list[i + 1], kw, cur);
     else
       solve_fixed(qs, t_list[i], t_list[i + 1], kw);
     if (qs->col_major) {

@@ -20,7 +20,7 @@ from __future__ import annotations
 
 import ctypes
 import weakref
-from concurrent.futures import ThreadPoolExecutor
+from concurrent.futures import ThreadPoolExecutor, wait
 from typing import Callable, Optional
 
 import numpy as np
@@ -448,22 +448,27 @@ class batch_solver:
         t = [float(x) for x in t_list]
         self._counts = [dict(rhs=0, attempts=0, accepted=0) for _ in self._parts]
         with ThreadPoolExecutor(len(self._parts)) as pool:  # sub-batches run concurrently (own streams)
-            for i in range(len(t) - 1):
+            # nobody looks at rho between the intervals without a callback: one solve covers them all
+            for i in range(len(t) - 1) if callback else range(min(1, len(t) - 1)):
                 if callback:
                     callback(t[i])
+                span = [t[i], t[i + 1]] if callback else t
                 subs = [self._gather(flat, ranges) for _, _, ranges, _ in self._parts]
-                futs = [pool.submit(part.solve, sub, [t[i], t[i + 1]], None, kwargs)
+                futs = [pool.submit(part.solve, sub, span, None, kwargs)
                         for (part, _, _, _), sub in zip(self._parts, subs)]
-                for f in futs:
-                    f.result()
-                for (_, _, ranges, _), sub in zip(self._parts, subs):
-                    self._scatter(flat, ranges, sub)
+                try:
+                    for f in futs:
+                        f.result()
+                finally:  # a sub-batch that failed holds its last good interval's state
+                    wait(futs)
+                    for (_, _, ranges, _), sub in zip(self._parts, subs):
+                        self._scatter(flat, ranges, sub)
                 self._count_interval()
         if callback and t:
             callback(t[-1])
 
     def _count_interval(self):
-        # each sub-batch solve covers one interval: its counters restart every interval
+        # a sub-batch's counters restart with every solve (one interval, or all without a callback)
         for c, (part, _, _, _) in zip(self._counts, self._parts):
             st = part.stats()
             for k in c:
@@ -480,11 +485,12 @@ class batch_solver:
         t = [float(x) for x in t_list]
         self._counts = [dict(rhs=0, attempts=0, accepted=0) for _ in self._parts]
         with ThreadPoolExecutor(len(self._parts)) as pool:  # sub-batches run concurrently (own streams)
-            for i in range(len(t) - 1):
+            for i in range(len(t) - 1) if callback else range(min(1, len(t) - 1)):
                 if callback:
                     callback(t[i])
-                futs = [pool.submit(part.solve_device, int(rho_ptr) + 16 * ranges[0][0], [t[i], t[i + 1]], None,
-                                    kwargs) for part, _, ranges, _ in self._parts]
+                span = [t[i], t[i + 1]] if callback else t
+                futs = [pool.submit(part.solve_device, int(rho_ptr) + 16 * ranges[0][0], span, None, kwargs)
+                        for part, _, ranges, _ in self._parts]
                 for f in futs:
                     f.result()
                 self._count_interval()

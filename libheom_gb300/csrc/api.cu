@@ -789,7 +789,18 @@ void build_model(heomgb_qme* q) {
   } else if (q->form == HEOMGB_HILB) {
     q->path = diag ? PATH_DIAG : PATH_GENERAL;
   } else {
-    q->path = PATH_LIOU;
+    if (rhs_smem_bytes(m, PATH_LIOU, false) > 200 * 1024)
+      throw unsupported_error("Liouville path supports n_level <= 56");
+    // heom_liou and heom_ado apply the operator of heom_hilb, written as
+    // superoperators (heom_liou.h:71-99): n^3 products per ADO and bath where
+    // the Hilbert-space form has n^2 (diagonal V) or 2 n^3 per matrix product.
+    // In FP64 the two agree to rounding, so the Hilbert-space kernels serve both
+    // (7-site depth 3, RK4: 23.2 us a stage as block-sparse products, 5.7 us as
+    // resident interval).  The mixed form keeps its own kernel: there the order
+    // of the FP32 sums shows.
+    const bool fits = diag ? diag_tile_smem(n2, K, 1, false) <= 200 * 1024
+                           : rhs_smem_bytes(m, PATH_GENERAL, false) <= 200 * 1024;
+    q->path = q->precision_eff == HEOMGB_FP64 && fits ? (diag ? PATH_DIAG : PATH_GENERAL) : PATH_LIOU;
   }
   if (q->path == PATH_DIAG) {
     // per-element active modes of the elementwise bath terms
@@ -959,9 +970,7 @@ void build_model(heomgb_qme* q) {
   } else if (q->path == PATH_GENERAL) {
     if (rhs_smem_bytes(m, PATH_GENERAL, false) > 200 * 1024)
       throw unsupported_error("general-V Hilbert path supports n_level <= 50");
-  } else {
-    if (rhs_smem_bytes(m, PATH_LIOU, false) > 200 * 1024)
-      throw unsupported_error("Liouville path supports n_level <= 56");
+  } else if (q->path == PATH_LIOU) {
     // superoperators (heom_liou.h:71-99)
     const cd I(0.0, 1.0), one(1.0, 0.0);
     Lil L;
@@ -1159,6 +1168,21 @@ ResidentArgs resident_args(heomgb_qme_solver* qs) {
 }
 Stage solver_stage(heomgb_qme_solver* qs);
 
+// The diagonal-coupling instances of the solver's models, concatenated.
+std::vector<DiagInst> solver_instances(const heomgb_qme_solver* qs) {
+  std::vector<DiagInst> insts;
+  long long off = 0;
+  for (heomgb_qme* m : qs->qmes) {
+    DiagInst I = m->dinst;
+    I.term_p = qs->term ? qs->tb.P : nullptr;
+    I.term_first = qs->term ? qs->tb.first : 0;
+    I.elem_off = off;
+    off += m->main_size();
+    insts.push_back(I);
+  }
+  return insts;
+}
+
 void alloc_solver(heomgb_qme_solver* qs) {
   heomgb_qme* q = qs->q;
   long long N = 0;
@@ -1193,8 +1217,15 @@ void alloc_solver(heomgb_qme_solver* qs) {
     if (qs->qmes.size() != 1) throw unsupported_error("the learned terminator is not available in batches");
     alloc_term(qs->arena, q, qs->tb);
   }
+  // a model that runs as resident intervals needs no tile search: its stage
+  // kernels (the fall-back, should the device not hold the cooperative grid) take
+  // the default shape
+  if (!std::getenv("HEOMGB_TILE")) plan_resident(qs);
   if (q->path == PATH_DIAG) {
-    autotune(qs);
+    if (qs->resident)
+      build_plan(qs->plan, solver_instances(qs), 128, 4, 1, qs->mixed, q->n_sm, qs->stream);
+    else
+      autotune(qs);
     qs->block = qs->plan.block;
     qs->grid = qs->plan.grid;
   } else {
@@ -1202,7 +1233,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
     qs->grid = rhs_grid_size(q->dm, q->path, qs->block, q->n_sm);
   }
   qs->partials = static_cast<double*>(A.alloc(sizeof(double) * std::max(qs->grid, 1)));
-  plan_resident(qs);
+  if (std::getenv("HEOMGB_TILE")) plan_resident(qs);
   plan_local(qs);
   plan_cluster(qs);
 }
@@ -1213,16 +1244,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
 void autotune(heomgb_qme_solver* qs) {
   const NvtxRange range("heomgb plan: tile search");
   heomgb_qme* q = qs->q;
-  std::vector<DiagInst> insts;
-  long long off = 0;
-  for (heomgb_qme* m : qs->qmes) {
-    DiagInst I = m->dinst;
-    I.term_p = qs->term ? qs->tb.P : nullptr;
-    I.term_first = qs->term ? qs->tb.first : 0;
-    I.elem_off = off;
-    off += m->main_size();
-    insts.push_back(I);
-  }
+  const std::vector<DiagInst> insts = solver_instances(qs);
   // Timed on a representative stage of the solver itself (its epilogue
   // traffic shapes the best tile as much as the right-hand side does) over
   // zeroed buffers with the controller idle (dt = 0): RK4 stage 2, an LSRK4
@@ -2407,7 +2429,7 @@ heomgb_status heomgb_qme_set_terminator(heomgb_qme* q, heomgb_mlp* mlp) {
     need_ready(q);
     if (q->live_solvers > 0) throw state_error("set_terminator: destroy the qme_solvers of this model first");
     if (mlp) {
-      if (q->path != PATH_DIAG) throw unsupported_error("the learned terminator needs diagonal couplings V (heom_hilb)");
+      if (q->path != PATH_DIAG || q->form != HEOMGB_HILB) throw unsupported_error("the learned terminator needs diagonal couplings V (heom_hilb)");
       if (q->sqrt_norm) throw unsupported_error("the learned terminator is trained for the integer normalisation");
       if (q->filter) throw unsupported_error("the learned terminator needs the complete truncated tier (no filter)");
       int din = 0, h = 0, dout = 0;
@@ -2588,7 +2610,7 @@ heomgb_status heomgb_batch_solver_create(heomgb_qme* const* qmes, int count, heo
     heomgb_qme* q0 = qmes[0];
     for (int i = 0; i < count; ++i) {
       need_ready(qmes[i]);
-      if (qmes[i]->path != PATH_DIAG)
+      if (qmes[i]->path != PATH_DIAG || qmes[i]->form != HEOMGB_HILB)
         throw unsupported_error("batches need heom_hilb models with diagonal couplings V");
       if (qmes[i]->precision_eff != q0->precision_eff)
         throw arg_error("batch models must share one effective precision (heomgb_qme_get_precision)");

@@ -344,6 +344,10 @@ struct heomgb_qme {
   int K = 0, n_hrchy = 0, path = PATH_DIAG;
   RhsModel dm{};
   DiagInst dinst{};          // diagonal-coupling instance (PATH_DIAG), device pointers into arena
+  // dense V with a common eigenbasis (FP64): the instance in that basis, for
+  // fixed-step solves, and the basis (null: none)
+  DiagInst rinst{};
+  const double2* rbasis = nullptr;
   DiagPlan diff_plan;        // tiles for calc_diff
   heomgb_mlp* term = nullptr;  // learned terminator (not owned); null = plain truncation
   const float2* term_cke = nullptr;  // its set-up tables (TermModel::cke, sgn), in term_arena
@@ -375,6 +379,8 @@ struct heomgb_qme_solver {
   bool mixed = false;
   bool separate = false;
   bool col_major = false;              // models store their ADOs column-major
+  bool rotated = false;                // works in the model's common eigenbasis of V (rinst)
+  int path = PATH_DIAG;                // of the stages: the model's, PATH_DIAG when rotated
   long long N = 0;
   DeviceArena arena;
   double2* otmp = nullptr;             // boundary transposes of col_major models
@@ -624,6 +630,215 @@ void filter_hierarchy(heomgb_qme* q, int K, int nh_full, cudaStream_t s, int*& n
   ck(cudaStreamSynchronize(s), "filtered tables");
 }
 
+// The diagonal-coupling instance of a model: H and the diagonals vd[u] of the
+// baths' V in the basis the instance works in (the caller's, or the rotated one),
+// with every table of the diagonal-coupling kernels on the device.
+DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vector<std::vector<cd>>& vd,
+                        const std::vector<int>& bath_ptr, const std::vector<cd>& sigma, const std::vector<cd>& sv,
+                        const std::vector<cd>& av, cudaStream_t s) {
+  const RhsModel& m = q->dm;
+  const int n = q->n, n2 = n * n, U = q->U, K = q->K, nh = q->n_hrchy;
+  // per-element active modes of the elementwise bath terms
+  std::vector<int> pp(n2 + 1, 0), pm(n2 + 1, 0), pmode, mmode;
+  std::vector<cd> cp, cmn, csd(n2, cd(0.0, 0.0));
+  const cd I(0.0, 1.0);
+  for (int a = 0; a < n; ++a)
+    for (int b = 0; b < n; ++b) {
+      const int e = a * n + b;
+      for (int u = 0; u < U; ++u) {
+        const cd sd = q->baths[u].sdelta;
+        const cd va = vd[u][a], vb = vd[u][b];
+        const cd cphi = I * (va - vb), cpsi = va + vb;
+        csd[e] += sd * (va - vb) * (va - vb);
+        for (int k = bath_ptr[u]; k < bath_ptr[u + 1]; ++k) {
+          const cd c1 = cphi * sigma[k];
+          if (c1 != cd(0.0, 0.0)) {
+            pmode.push_back(k);
+            cp.push_back(c1);
+          }
+          const cd c2 = cphi * sv[k] - cpsi * av[k];
+          if (c2 != cd(0.0, 0.0)) {
+            mmode.push_back(k);
+            cmn.push_back(c2);
+          }
+        }
+      }
+      pp[e + 1] = static_cast<int>(pmode.size());
+      pm[e + 1] = static_cast<int>(mmode.size());
+    }
+  DiagInst di{};
+  int max_terms = 0, sum_terms = 0;
+  for (int e = 0; e < n2; ++e) {
+    max_terms = std::max({max_terms, pp[e + 1] - pp[e], pm[e + 1] - pm[e]});
+    sum_terms = std::max(sum_terms, pp[e + 1] - pp[e] + pm[e + 1] - pm[e]);
+  }
+  di.plus_ptr = q->arena.upload(pp, s);
+  di.plus_mode = q->arena.upload(pmode, s);
+  di.minus_ptr = q->arena.upload(pm, s);
+  di.minus_mode = q->arena.upload(mmode, s);
+  di.c_plus = q->arena.upload(to_d2(cp), s);
+  di.c_minus = q->arena.upload(to_d2(cmn), s);
+  di.c_plus_f = q->arena.upload(to_f2(cp), s);
+  di.c_minus_f = q->arena.upload(to_f2(cmn), s);
+  di.c_sd = q->arena.upload(to_d2(csd), s);
+  di.c_sd_f = q->arena.upload(to_f2(csd), s);
+  di.n = n;
+  di.n2 = n2;
+  di.K = K;
+  di.nh = nh;
+  bool h_real = true;
+  for (const cd& v : H) h_real = h_real && v.imag() == 0.0;
+  di.h_real = h_real ? 1 : 0;
+  {
+    bool sym = h_real;
+    for (int a = 0; a < n && sym; ++a)
+      for (int b = 0; b < a && sym; ++b) sym = H[static_cast<size_t>(a) * n + b] == H[static_cast<size_t>(b) * n + a];
+    di.h_sym = sym ? 1 : 0;
+  }
+  di.sqrt_norm = m.sqrt_norm;
+  di.max_terms = max_terms;
+  di.sum_terms = sum_terms;
+  {
+    std::vector<int> eo(n2);
+    for (int e = 0; e < n2; ++e) eo[e] = e;
+    std::stable_sort(eo.begin(), eo.end(),
+                     [&](int x, int y) { return pp[x + 1] - pp[x] + pm[x + 1] - pm[x] > pp[y + 1] - pp[y] + pm[y + 1] - pm[y]; });
+    di.e_order = q->arena.upload(eo, s);
+  }
+  di.elem_off = 0;
+  di.p1 = m.p1;
+  di.m1 = m.m1;
+  di.nidx = m.nidx;
+  di.ngd = m.ngd;
+  di.ngd_f = m.ngd_f;
+  di.H = q->arena.upload(to_d2(H), s);
+  di.H_f = q->arena.upload(to_f2(H), s);
+  int* plus_any = static_cast<int*>(q->arena.alloc(sizeof(int) * std::max(nh, 1)));
+  if (K > 0)
+    ck(launch_plus_any(K, nh, m.p1, plus_any, s), "plus_any");
+  else
+    ck(cudaMemsetAsync(plus_any, 0, sizeof(int) * std::max(nh, 1), s), "memset");
+  di.plus_any = plus_any;
+  // the FP64 coefficients scaled by every occupation (the FP64 kernels' per-term products, tabulated)
+  di.occ_rows = q->max_depth + 1;
+  const int n_plus = static_cast<int>(cp.size()), n_minus = static_cast<int>(cmn.size());
+  double2* cmn_n = static_cast<double2*>(q->arena.alloc(sizeof(double2) * std::max<size_t>(1, static_cast<size_t>(n_minus) * di.occ_rows)));
+  ck(launch_scaled_coef(n_minus, di.occ_rows, di.c_minus, cmn_n, false, m.sqrt_norm != 0, s), "scaled coefficients");
+  di.c_minus_n = cmn_n;
+  di.c_plus_n = nullptr;
+  if (m.sqrt_norm) {
+    double2* cp_n = static_cast<double2*>(q->arena.alloc(sizeof(double2) * std::max<size_t>(1, static_cast<size_t>(n_plus) * di.occ_rows)));
+    ck(launch_scaled_coef(n_plus, di.occ_rows, di.c_plus, cp_n, true, true, s), "scaled coefficients");
+    di.c_plus_n = cp_n;
+  }
+  // site-local baths (every V_u diagonal with a single nonzero entry, at site
+  // s_u): the -1 coefficients of an element in the row, column or diagonal
+  // of s_u, formed as the per-element table above forms them, and the
+  // per-ADO records of occupied modes (k_rhs_sites)
+  {
+    std::vector<int> usite(U, -1);
+    bool site_local = U > 0 && K > 0;
+    for (int u = 0; u < U && site_local; ++u) {
+      int cnt = 0;
+      for (int a = 0; a < n; ++a)
+        if (vd[u][a] != cd(0.0, 0.0)) {
+          ++cnt;
+          usite[u] = a;
+        }
+      site_local = cnt == 1;
+    }
+    if (site_local) {
+      std::vector<int> msite(K, 0);
+      std::vector<cd> cm3(3 * static_cast<size_t>(K));
+      for (int u = 0; u < U; ++u) {
+        const cd v = vd[u][usite[u]], zero(0.0, 0.0);
+        const cd vas[3] = {v, zero, v}, vbs[3] = {zero, v, v};  // row, column, diagonal of the site
+        for (int k = bath_ptr[u]; k < bath_ptr[u + 1]; ++k) {
+          msite[k] = usite[u];
+          for (int c = 0; c < 3; ++c) {
+            const cd cphi = I * (vas[c] - vbs[c]), cpsi = vas[c] + vbs[c];
+            cm3[3 * static_cast<size_t>(k) + c] = cphi * sv[k] - cpsi * av[k];
+          }
+        }
+      }
+      // the +1 coefficient i (v_a - v_b) sigma_k for the row and column cases, and
+      // the modes of every site in increasing k
+      std::vector<cd> cp2(2 * static_cast<size_t>(K));
+      std::vector<int> sptr(n + 1, 0), smodes;
+      for (int u = 0; u < U; ++u) {
+        const cd v = vd[u][usite[u]], zero(0.0, 0.0);
+        for (int k = bath_ptr[u]; k < bath_ptr[u + 1]; ++k) {
+          cp2[2 * static_cast<size_t>(k)] = I * (v - zero) * sigma[k];
+          cp2[2 * static_cast<size_t>(k) + 1] = I * (zero - v) * sigma[k];
+        }
+      }
+      for (int site = 0; site < n; ++site) {
+        for (int k = 0; k < K; ++k)
+          if (msite[k] == site) smodes.push_back(k);
+        sptr[site + 1] = static_cast<int>(smodes.size());
+      }
+      di.site_local = 1;
+      di.site_w = std::max(1, std::min(K, q->max_depth));
+      const int* dms = q->arena.upload(msite, s);
+      di.site_cm3 = q->arena.upload(to_f2(cm3), s);
+      di.site_cp2 = q->arena.upload(to_f2(cp2), s);
+      di.site_cm3_d = q->arena.upload(to_d2(cm3), s);
+      di.site_cp2_d = q->arena.upload(to_d2(cp2), s);
+      di.site_ptr = q->arena.upload(sptr, s);
+      di.site_modes = q->arena.upload(smodes, s);
+      int4* rec = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
+      di.site_rec = rec;
+      ck(launch_site_records(di, dms, rec, s), "site records");
+      ck(cudaStreamSynchronize(s), "site records sync");
+    }
+  }
+  return di;
+}
+
+// A basis in which every V_u is diagonal: W with W^dagger V_u W = diag(vd[u]),
+// where the V_u are Hermitian and commute (one bath always does).  The
+// eigenvectors of a fixed combination of them, checked on each; eigenvalues
+// that agree to rounding are made equal, so that no term hangs on their
+// difference.
+bool common_basis(const heomgb_qme* q, std::vector<cd>& W, std::vector<std::vector<cd>>& vd) {
+  const int n = q->n, n2 = n * n;
+  std::vector<cd> M(n2, cd(0.0, 0.0));
+  std::vector<double> top(q->U, 0.0);
+  double w = 1.0;
+  for (int u = 0; u < q->U; ++u, w *= 0.618033988749895) {
+    const std::vector<cd>& V = q->baths[u].V;
+    for (const cd& v : V) top[u] = std::max(top[u], std::abs(v));
+    if (!(top[u] > 0.0) || !std::isfinite(top[u])) return false;
+    for (int a = 0; a < n; ++a)
+      for (int b = 0; b < n; ++b) {
+        if (std::abs(V[a * n + b] - std::conj(V[b * n + a])) > 1e-15 * top[u]) return false;
+        M[a * n + b] += w / top[u] * V[a * n + b];
+      }
+  }
+  std::vector<double> ev;
+  hermitian_eigen(M, n, ev, W);
+  vd.assign(q->U, std::vector<cd>(n));
+  for (int u = 0; u < q->U; ++u) {
+    const std::vector<cd>& V = q->baths[u].V;
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j) {
+        cd acc(0.0, 0.0);
+        for (int a = 0; a < n; ++a)
+          for (int b = 0; b < n; ++b) acc += std::conj(W[a * n + i]) * V[a * n + b] * W[b * n + j];
+        if (i == j)
+          vd[u][i] = cd(acc.real(), 0.0);
+        else if (std::abs(acc) > 1e-14 * top[u])
+          return false;
+      }
+    for (int i = 0; i < n; ++i) {
+      if (std::abs(vd[u][i]) <= 1e-14 * top[u]) vd[u][i] = cd(0.0, 0.0);
+      for (int j = 0; j < i; ++j)
+        if (std::abs(vd[u][i] - vd[u][j]) <= 1e-14 * top[u]) vd[u][i] = vd[u][j];
+    }
+  }
+  return true;
+}
+
 void build_model(heomgb_qme* q) {
   if (q->n <= 0) throw state_error("set_param: Hamiltonian not set");
   if (q->U < 0) throw state_error("set_param: alloc_noises not called");
@@ -636,6 +851,7 @@ void build_model(heomgb_qme* q) {
   q->term = nullptr;  // a rebuilt model starts with plain truncation
   q->diff_tb = TermBuffers{};
   q->ready = false;
+  q->rbasis = nullptr;
   cudaStream_t s = q->stream();
   const int n = q->n, n2 = n * n, U = q->U;
   // linear mode index lk (heom.h:65-74) and per-mode coefficients
@@ -803,173 +1019,35 @@ void build_model(heomgb_qme* q) {
     q->path = q->precision_eff == HEOMGB_FP64 && fits ? (diag ? PATH_DIAG : PATH_GENERAL) : PATH_LIOU;
   }
   if (q->path == PATH_DIAG) {
-    // per-element active modes of the elementwise bath terms
-    std::vector<int> pp(n2 + 1, 0), pm(n2 + 1, 0), pmode, mmode;
-    std::vector<cd> cp, cmn, csd(n2, cd(0.0, 0.0));
-    const cd I(0.0, 1.0);
-    for (int a = 0; a < n; ++a)
-      for (int b = 0; b < n; ++b) {
-        const int e = a * n + b;
-        for (int u = 0; u < U; ++u) {
-          const Bath& B = q->baths[u];
-          const cd va = B.V[static_cast<size_t>(a) * n + a], vb = B.V[static_cast<size_t>(b) * n + b];
-          const cd cphi = I * (va - vb), cpsi = va + vb;
-          csd[e] += B.sdelta * (va - vb) * (va - vb);
-          for (int k = bath_ptr[u]; k < bath_ptr[u + 1]; ++k) {
-            const cd c1 = cphi * sigma[k];
-            if (c1 != cd(0.0, 0.0)) {
-              pmode.push_back(k);
-              cp.push_back(c1);
-            }
-            const cd c2 = cphi * sv[k] - cpsi * av[k];
-            if (c2 != cd(0.0, 0.0)) {
-              mmode.push_back(k);
-              cmn.push_back(c2);
-            }
-          }
-        }
-        pp[e + 1] = static_cast<int>(pmode.size());
-        pm[e + 1] = static_cast<int>(mmode.size());
-      }
-    int max_terms = 0, sum_terms = 0;
-    for (int e = 0; e < n2; ++e) {
-      max_terms = std::max({max_terms, pp[e + 1] - pp[e], pm[e + 1] - pm[e]});
-      sum_terms = std::max(sum_terms, pp[e + 1] - pp[e] + pm[e + 1] - pm[e]);
-    }
-    m.plus_ptr = q->arena.upload(pp, s);
-    m.plus_mode = q->arena.upload(pmode, s);
-    m.minus_ptr = q->arena.upload(pm, s);
-    m.minus_mode = q->arena.upload(mmode, s);
-    m.c_plus = q->arena.upload(to_d2(cp), s);
-    m.c_minus = q->arena.upload(to_d2(cmn), s);
-    m.c_plus_f = q->arena.upload(to_f2(cp), s);
-    m.c_minus_f = q->arena.upload(to_f2(cmn), s);
-    m.c_sd = q->arena.upload(to_d2(csd), s);
-    m.c_sd_f = q->arena.upload(to_f2(csd), s);
-    DiagInst& di = q->dinst;
-    di = DiagInst{};
-    di.n = n;
-    di.n2 = n2;
-    di.K = K;
-    di.nh = nh;
-    di.h_real = m.h_real;
-    {
-      bool sym = m.h_real != 0;
-      for (int a = 0; a < n && sym; ++a)
-        for (int b = 0; b < a && sym; ++b) sym = q->H[static_cast<size_t>(a) * n + b] == q->H[static_cast<size_t>(b) * n + a];
-      di.h_sym = sym ? 1 : 0;
-    }
-    di.sqrt_norm = m.sqrt_norm;
-    di.max_terms = max_terms;
-    di.sum_terms = sum_terms;
-    {
-      std::vector<int> eo(n2);
-      for (int e = 0; e < n2; ++e) eo[e] = e;
-      std::stable_sort(eo.begin(), eo.end(),
-                       [&](int x, int y) { return pp[x + 1] - pp[x] + pm[x + 1] - pm[x] > pp[y + 1] - pp[y] + pm[y + 1] - pm[y]; });
-      di.e_order = q->arena.upload(eo, s);
-    }
-    di.elem_off = 0;
-    di.p1 = m.p1;
-    di.m1 = m.m1;
-    di.nidx = m.nidx;
-    di.ngd = m.ngd;
-    di.ngd_f = m.ngd_f;
-    di.H = m.H;
-    di.H_f = m.H_f;
-    di.plus_ptr = m.plus_ptr;
-    di.plus_mode = m.plus_mode;
-    di.minus_ptr = m.minus_ptr;
-    di.minus_mode = m.minus_mode;
-    di.c_plus = m.c_plus;
-    di.c_minus = m.c_minus;
-    di.c_plus_f = m.c_plus_f;
-    di.c_minus_f = m.c_minus_f;
-    di.c_sd = m.c_sd;
-    di.c_sd_f = m.c_sd_f;
-    int* plus_any = static_cast<int*>(q->arena.alloc(sizeof(int) * std::max(nh, 1)));
-    if (K > 0)
-      ck(launch_plus_any(K, nh, m.p1, plus_any, s), "plus_any");
-    else
-      ck(cudaMemsetAsync(plus_any, 0, sizeof(int) * std::max(nh, 1), s), "memset");
-    di.plus_any = plus_any;
-    // the FP64 coefficients scaled by every occupation (the FP64 kernels' per-term products, tabulated)
-    di.occ_rows = q->max_depth + 1;
-    const int n_plus = static_cast<int>(cp.size()), n_minus = static_cast<int>(cmn.size());
-    double2* cmn_n = static_cast<double2*>(q->arena.alloc(sizeof(double2) * std::max<size_t>(1, static_cast<size_t>(n_minus) * di.occ_rows)));
-    ck(launch_scaled_coef(n_minus, di.occ_rows, m.c_minus, cmn_n, false, m.sqrt_norm != 0, s), "scaled coefficients");
-    di.c_minus_n = cmn_n;
-    di.c_plus_n = nullptr;
-    if (m.sqrt_norm) {
-      double2* cp_n = static_cast<double2*>(q->arena.alloc(sizeof(double2) * std::max<size_t>(1, static_cast<size_t>(n_plus) * di.occ_rows)));
-      ck(launch_scaled_coef(n_plus, di.occ_rows, m.c_plus, cp_n, true, true, s), "scaled coefficients");
-      di.c_plus_n = cp_n;
-    }
-    // site-local baths (every V_u diagonal with a single nonzero entry, at site
-    // s_u): the -1 coefficients of an element in the row, column or diagonal
-    // of s_u, formed as the per-element table above forms them, and the
-    // per-ADO records of occupied modes (k_rhs_sites)
-    {
-      std::vector<int> usite(U, -1);
-      bool site_local = U > 0 && K > 0;
-      for (int u = 0; u < U && site_local; ++u) {
-        int cnt = 0;
-        for (int a = 0; a < n; ++a)
-          if (q->baths[u].V[static_cast<size_t>(a) * n + a] != cd(0.0, 0.0)) {
-            ++cnt;
-            usite[u] = a;
-          }
-        site_local = cnt == 1;
-      }
-      if (site_local) {
-        std::vector<int> msite(K, 0);
-        std::vector<cd> cm3(3 * static_cast<size_t>(K));
-        for (int u = 0; u < U; ++u) {
-          const cd v = q->baths[u].V[static_cast<size_t>(usite[u]) * n + usite[u]], zero(0.0, 0.0);
-          const cd vas[3] = {v, zero, v}, vbs[3] = {zero, v, v};  // row, column, diagonal of the site
-          for (int k = bath_ptr[u]; k < bath_ptr[u + 1]; ++k) {
-            msite[k] = usite[u];
-            for (int c = 0; c < 3; ++c) {
-              const cd cphi = I * (vas[c] - vbs[c]), cpsi = vas[c] + vbs[c];
-              cm3[3 * static_cast<size_t>(k) + c] = cphi * sv[k] - cpsi * av[k];
-            }
-          }
-        }
-        // the +1 coefficient i (v_a - v_b) sigma_k for the row and column cases, and
-        // the modes of every site in increasing k
-        std::vector<cd> cp2(2 * static_cast<size_t>(K));
-        std::vector<int> sptr(n + 1, 0), smodes;
-        for (int u = 0; u < U; ++u) {
-          const cd v = q->baths[u].V[static_cast<size_t>(usite[u]) * n + usite[u]], zero(0.0, 0.0);
-          for (int k = bath_ptr[u]; k < bath_ptr[u + 1]; ++k) {
-            cp2[2 * static_cast<size_t>(k)] = I * (v - zero) * sigma[k];
-            cp2[2 * static_cast<size_t>(k) + 1] = I * (zero - v) * sigma[k];
-          }
-        }
-        for (int site = 0; site < n; ++site) {
-          for (int k = 0; k < K; ++k)
-            if (msite[k] == site) smodes.push_back(k);
-          sptr[site + 1] = static_cast<int>(smodes.size());
-        }
-        di.site_local = 1;
-        di.site_w = std::max(1, std::min(K, q->max_depth));
-        const int* dms = q->arena.upload(msite, s);
-        di.site_cm3 = q->arena.upload(to_f2(cm3), s);
-        di.site_cp2 = q->arena.upload(to_f2(cp2), s);
-        di.site_cm3_d = q->arena.upload(to_d2(cm3), s);
-        di.site_cp2_d = q->arena.upload(to_d2(cp2), s);
-        di.site_ptr = q->arena.upload(sptr, s);
-        di.site_modes = q->arena.upload(smodes, s);
-        int4* rec = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
-        di.site_rec = rec;
-        ck(launch_site_records(di, dms, rec, s), "site records");
-        ck(cudaStreamSynchronize(s), "site records sync");
-      }
-    }
-    build_plan(q->diff_plan, {di}, 128, 4, 1, q->precision_eff == HEOMGB_MIXED, q->n_sm, s);
+    std::vector<std::vector<cd>> vd(U, std::vector<cd>(n));
+    for (int u = 0; u < U; ++u)
+      for (int a = 0; a < n; ++a) vd[u][a] = q->baths[u].V[static_cast<size_t>(a) * n + a];
+    q->dinst = make_diag_inst(q, q->H, vd, bath_ptr, sigma, sv, av, s);
+    build_plan(q->diff_plan, {q->dinst}, 128, 4, 1, q->precision_eff == HEOMGB_MIXED, q->n_sm, s);
   } else if (q->path == PATH_GENERAL) {
     if (rhs_smem_bytes(m, PATH_GENERAL, false) > 200 * 1024)
       throw unsupported_error("general-V Hilbert path supports n_level <= 50");
+    // FP64 models whose V_u share an eigenbasis: fixed-step solves (linear in the
+    // state, so a change of basis commutes with them) run there on the
+    // diagonal-coupling kernels, which drop the n-term products of every bath
+    // and reach the resident plans (two levels, V = sigma_x, depth 10: 9.7 us a
+    // stage in k_rhs_general, 2.1 in the basis; the state's way in and out adds
+    // one k_rotate each).  The mixed form stays: its FP32 rounding depends on
+    // the basis.
+    std::vector<cd> W;
+    std::vector<std::vector<cd>> vd;
+    if (q->precision_eff == HEOMGB_FP64 && U > 0 && common_basis(q, W, vd) &&
+        diag_tile_smem(n2, K, 1, false) <= 200 * 1024) {
+      std::vector<cd> Hr(n2, cd(0.0, 0.0)), T(n2, cd(0.0, 0.0));
+      for (int a = 0; a < n; ++a)
+        for (int b = 0; b < n; ++b)
+          for (int j = 0; j < n; ++j) T[a * n + j] += q->H[a * n + b] * W[b * n + j];
+      for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j)
+          for (int a = 0; a < n; ++a) Hr[i * n + j] += std::conj(W[a * n + i]) * T[a * n + j];
+      q->rinst = make_diag_inst(q, Hr, vd, bath_ptr, sigma, sv, av, s);
+      q->rbasis = q->arena.upload(to_d2(W), s);
+    }
   } else if (q->path == PATH_LIOU) {
     // superoperators (heom_liou.h:71-99)
     const cd I(0.0, 1.0), one(1.0, 0.0);
@@ -1122,6 +1200,9 @@ void plan_resident(heomgb_qme_solver* qs);
 void plan_local(heomgb_qme_solver* qs);
 void plan_cluster(heomgb_qme_solver* qs);
 
+// The model's instance in the basis that the solver works in.
+const DiagInst& solver_inst(const heomgb_qme_solver* qs) { return qs->rotated ? qs->q->rinst : qs->q->dinst; }
+
 // The resident kernel of the solver's scheme.
 int resident_scheme(const heomgb_qme_solver* qs) {
   return qs->kind == HEOMGB_RK4 ? kResidentRk4 : qs->kind == HEOMGB_LSRK4 ? kResidentLs : kResidentDp;
@@ -1134,14 +1215,14 @@ int resident_variant(const heomgb_qme_solver* qs) {
   if (qs->mixed) return scheme;
   if (scheme == kResidentRk4) return kResidentRk4F64;
   // the FP64 Dormand-Prince interval reads the site-local records
-  if (scheme == kResidentDp && qs->q->dinst.site_local && qs->q->dinst.site_rec) return kResidentDpF64;
+  if (scheme == kResidentDp && solver_inst(qs).site_local && solver_inst(qs).site_rec) return kResidentDpF64;
   return -1;
 }
 
 // Arguments of the resident kernels for the solver's buffers and its tuned shape.
 ResidentArgs resident_args(heomgb_qme_solver* qs) {
   ResidentArgs a{};
-  a.inst = qs->q->dinst;
+  a.inst = solver_inst(qs);
   a.ctl = qs->ctl;
   for (int i = 0; i < 2; ++i) {
     a.S[i] = qs->S[i];
@@ -1173,7 +1254,7 @@ std::vector<DiagInst> solver_instances(const heomgb_qme_solver* qs) {
   std::vector<DiagInst> insts;
   long long off = 0;
   for (heomgb_qme* m : qs->qmes) {
-    DiagInst I = m->dinst;
+    DiagInst I = qs->rotated ? m->rinst : m->dinst;
     I.term_p = qs->term ? qs->tb.P : nullptr;
     I.term_first = qs->term ? qs->tb.first : 0;
     I.elem_off = off;
@@ -1189,6 +1270,8 @@ void alloc_solver(heomgb_qme_solver* qs) {
   for (heomgb_qme* m : qs->qmes) N += m->main_size();
   qs->N = N;
   qs->mixed = q->precision_eff == HEOMGB_MIXED;
+  qs->rotated = q->rbasis && qs->kind != HEOMGB_RKDP;  // the error norm is not invariant
+  qs->path = qs->rotated ? PATH_DIAG : q->path;
   qs->col_major = q->col_major != 0;
   qs->separate = qs->mixed;
   const size_t bd = sizeof(double2) * N;
@@ -1204,7 +1287,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
     qs->Ytmp[1] = A.alloc(bb);
   }
   if (qs->kind == HEOMGB_RK4 || qs->kind == HEOMGB_LSRK4) qs->acc = static_cast<double2*>(A.alloc(bd));
-  if (qs->col_major) qs->otmp = static_cast<double2*>(A.alloc(bd));
+  if (qs->col_major || qs->rotated) qs->otmp = static_cast<double2*>(A.alloc(bd));
   if (qs->kind == HEOMGB_RKDP)
     for (int i = 0; i < 6; ++i) qs->K[i] = A.alloc(bb);
   qs->ctl = static_cast<DpCtl*>(A.alloc(sizeof(DpCtl)));
@@ -1221,7 +1304,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
   // kernels (the fall-back, should the device not hold the cooperative grid) take
   // the default shape
   if (!std::getenv("HEOMGB_TILE")) plan_resident(qs);
-  if (q->path == PATH_DIAG) {
+  if (qs->path == PATH_DIAG) {
     if (qs->resident)
       build_plan(qs->plan, solver_instances(qs), 128, 4, 1, qs->mixed, q->n_sm, qs->stream);
     else
@@ -1229,8 +1312,8 @@ void alloc_solver(heomgb_qme_solver* qs) {
     qs->block = qs->plan.block;
     qs->grid = qs->plan.grid;
   } else {
-    qs->block = rhs_block_size(q->dm, q->path);
-    qs->grid = rhs_grid_size(q->dm, q->path, qs->block, q->n_sm);
+    qs->block = rhs_block_size(q->dm, qs->path);
+    qs->grid = rhs_grid_size(q->dm, qs->path, qs->block, q->n_sm);
   }
   qs->partials = static_cast<double*>(A.alloc(sizeof(double) * std::max(qs->grid, 1)));
   if (std::getenv("HEOMGB_TILE")) plan_resident(qs);
@@ -1455,14 +1538,14 @@ void plan_resident(heomgb_qme_solver* qs) {
   qs->resident = false;
   const int scheme = resident_scheme(qs);
   const int variant = resident_variant(qs);
-  if (variant < 0 || q->path != PATH_DIAG || qs->qmes.size() != 1 || qs->term) return;
-  if (q->dinst.max_terms > kResidentTerms / 2) return;  // the per-element term table holds 4 + 4
+  if (variant < 0 || qs->path != PATH_DIAG || qs->qmes.size() != 1 || qs->term) return;
+  if (solver_inst(qs).max_terms > kResidentTerms / 2) return;  // the per-element term table holds 4 + 4
   if (const char* env = std::getenv("HEOMGB_RESIDENT"))
     if (std::string(env) == "0") return;
   int coop = 0;
   ck(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, q->device), "device attribute");
   if (!coop) return;
-  const DiagInst& I = q->dinst;
+  const DiagInst& I = solver_inst(qs);
   const bool hreal = I.h_real != 0;
   int pin = 0;
   if (const char* env = std::getenv("HEOMGB_RESIDENT_PER_SM")) pin = std::atoi(env);
@@ -1567,7 +1650,7 @@ void plan_local(heomgb_qme_solver* qs) {
   const NvtxRange range("heomgb plan: instance-resident bins");
   heomgb_qme* q = qs->q;
   qs->local = false;
-  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || q->path != PATH_DIAG || qs->term || qs->plan.tcore)
+  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || qs->path != PATH_DIAG || qs->term || qs->plan.tcore)
     return;
   const int scheme = resident_scheme(qs);
   if (qs->resident && qs->res_step_ms <= 0.f) return;  // an untimed (pinned) resident plan stays
@@ -1710,9 +1793,8 @@ void plan_local(heomgb_qme_solver* qs) {
 // pinned by HEOMGB_TILE, HEOMGB_RESIDENT or HEOMGB_LOCAL stays.
 void plan_cluster(heomgb_qme_solver* qs) {
   const NvtxRange range("heomgb plan: cluster-resident bins");
-  heomgb_qme* q = qs->q;
   qs->cluster = false;
-  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || q->path != PATH_DIAG || qs->term) return;
+  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || qs->path != PATH_DIAG || qs->term) return;
   bool force = false;
   if (const char* env = std::getenv("HEOMGB_CLUSTER")) {
     if (std::string(env) == "0") return;
@@ -1886,8 +1968,8 @@ void launch_stage(heomgb_qme_solver* qs, const Stage& st) {
     in.ctl = st.ctl;
     ck(term_enqueue(qs->term, qs->tb, term_model(qs->q), in, qs->mixed, qs->stream), "terminator");
   }
-  const bool diag = qs->q->path == PATH_DIAG;
-  ck(launch_rhs(qs->q->dm, diag ? &qs->plan.ds : nullptr, st, qs->q->path, qs->mixed, false, qs->grid, qs->block,
+  const bool diag = qs->path == PATH_DIAG;
+  ck(launch_rhs(qs->q->dm, diag ? &qs->plan.ds : nullptr, st, qs->path, qs->mixed, false, qs->grid, qs->block,
                 qs->stream),
      "stage launch");
 }
@@ -2069,7 +2151,7 @@ void solve_fixed(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwarg
     a.dt_step = dt;
     a.dt_last = last;
     busy_begin(qs);
-    const cudaError_t le = launch_resident(a, resident_variant(qs), qs->q->dinst.h_real != 0, qs->res_ept,
+    const cudaError_t le = launch_resident(a, resident_variant(qs), solver_inst(qs).h_real != 0, qs->res_ept,
                                            qs->res_grid, qs->res_block, qs->res_smem, qs->stream);
     if (le != cudaErrorCooperativeLaunchTooLarge) {
       ck(le, "resident interval");
@@ -2125,7 +2207,7 @@ int solve_resident(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwa
   ck(launch_ctl_init(qs->ctl, t0, dt, t1, atol, rtol, cur, qs->stream), "ctl init");
   ck(cudaMemsetAsync(qs->res_bar, 0, kResidentBarWords * sizeof(unsigned long long), qs->stream), "barrier reset");
   busy_begin(qs);
-  const cudaError_t le = launch_resident(resident_args(qs), resident_variant(qs), qs->q->dinst.h_real != 0, qs->res_ept,
+  const cudaError_t le = launch_resident(resident_args(qs), resident_variant(qs), solver_inst(qs).h_real != 0, qs->res_ept,
                                          qs->res_grid, qs->res_block, qs->res_smem, qs->stream);
   if (le == cudaErrorCooperativeLaunchTooLarge) {
     // the device cannot hold the grid now (another context holds SMs or
@@ -2229,7 +2311,12 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
       cb(t_list[i], user);
     }
     if (i == 0 || cb) {
-      if (qs->col_major) {  // the caller's ADOs are column-major: transpose at the boundary
+      if (qs->rotated) {
+        ck(cudaMemcpyAsync(qs->otmp, rho, bytes, in_kind, qs->stream), "state in");
+        ck(launch_rotate(qs->otmp, qs->S[0], qs->q->rbasis, qs->q->n, qs->q->n_hrchy, true, qs->col_major, false,
+                         qs->stream),
+           "rotate in");
+      } else if (qs->col_major) {  // the caller's ADOs are column-major: transpose at the boundary
         ck(cudaMemcpyAsync(qs->otmp, rho, bytes, in_kind, qs->stream), "state in");
         transpose_instances(qs, qs->otmp, qs->S[0]);
       } else {
@@ -2243,7 +2330,12 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
                          : solve_adaptive(qs, t_list[i], t_list[i + 1], kw, cur);
     else
       solve_fixed(qs, t_list[i], t_list[i + 1], kw);
-    if (qs->col_major) {
+    if (qs->rotated) {
+      ck(launch_rotate(qs->S[cur], qs->otmp, qs->q->rbasis, qs->q->n, qs->q->n_hrchy, false, false, qs->col_major,
+                       qs->stream),
+         "rotate out");
+      ck(cudaMemcpyAsync(rho, qs->otmp, bytes, out_kind, qs->stream), "state out");
+    } else if (qs->col_major) {
       transpose_instances(qs, qs->S[cur], qs->otmp);
       ck(cudaMemcpyAsync(rho, qs->otmp, bytes, out_kind, qs->stream), "state out");
     } else {
@@ -2653,7 +2745,7 @@ heomgb_status heomgb_qme_solver_tuning(const heomgb_qme_solver* qs, int* block, 
                                        int* n_tiles, int* min_blocks) {
   return guard([&] {
     require(qs != nullptr, "null qme_solver");
-    const bool diag = qs->q->path == PATH_DIAG;
+    const bool diag = qs->path == PATH_DIAG;
     if (block) *block = qs->block;
     if (elems_per_thread) *elems_per_thread = diag ? qs->plan.ept : 0;
     if (n_tiles) *n_tiles = diag ? qs->plan.ds.n_tiles : 0;
@@ -2692,7 +2784,7 @@ heomgb_status heomgb_qme_solver_local(const heomgb_qme_solver* qs, int* on, int*
 heomgb_status heomgb_qme_solver_site_kernel(const heomgb_qme_solver* qs, int* on, int* ados_per_tile) {
   return guard([&] {
     require(qs != nullptr && on != nullptr, "null argument");
-    const bool sites = qs->q->path == PATH_DIAG && qs->plan.sites;
+    const bool sites = qs->path == PATH_DIAG && qs->plan.sites;
     *on = sites ? 1 : 0;
     if (ados_per_tile) *ados_per_tile = sites ? qs->plan.ds.sites_tile : 0;
   });
@@ -2701,7 +2793,7 @@ heomgb_status heomgb_qme_solver_site_kernel(const heomgb_qme_solver* qs, int* on
 heomgb_status heomgb_qme_solver_tensor_cores(const heomgb_qme_solver* qs, int* on) {
   return guard([&] {
     require(qs != nullptr && on != nullptr, "null argument");
-    *on = (qs->q->path == PATH_DIAG && qs->plan.tcore) ? 1 : 0;
+    *on = (qs->path == PATH_DIAG && qs->plan.tcore) ? 1 : 0;
   });
 }
 

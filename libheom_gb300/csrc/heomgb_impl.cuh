@@ -47,20 +47,6 @@ struct RhsModel {
   const float2* ngd_f;
   const double2* H;                 // n2
   const float2* H_f;
-  // diagonal-V path: per element e=(a,b), the modes whose bath couples e,
-  // with nonzero coefficients only:
-  //   +1 term  c_plus  = i(v_a - v_b) sigma_k                      (plus_ptr/plus_mode)
-  //   -1 term  c_minus = i(v_a - v_b) s_k - (v_a + v_b) a_k, x n_k  (minus_ptr/minus_mode)
-  const int* plus_ptr;              // n2+1
-  const int* plus_mode;
-  const int* minus_ptr;             // n2+1
-  const int* minus_mode;
-  const double2* c_plus;
-  const double2* c_minus;
-  const float2* c_plus_f;
-  const float2* c_minus_f;
-  const double2* c_sd;              // n2: sum_u s_delta_u (v_ua - v_ub)^2
-  const float2* c_sd_f;
   // general-V and Liouville paths
   const double2* V;                 // U*n2
   const float2* V_f;
@@ -133,15 +119,19 @@ struct DiagInst {
   const float2* ngd_f;
   const double2* H;
   const float2* H_f;
-  const int* plus_ptr;
+  // diagonal-V path: per element e=(a,b), the modes whose bath couples e,
+  // with nonzero coefficients only:
+  //   +1 term  c_plus  = i(v_a - v_b) sigma_k                      (plus_ptr/plus_mode)
+  //   -1 term  c_minus = i(v_a - v_b) s_k - (v_a + v_b) a_k, x n_k  (minus_ptr/minus_mode)
+  const int* plus_ptr;              // n2+1
   const int* plus_mode;
-  const int* minus_ptr;
+  const int* minus_ptr;             // n2+1
   const int* minus_mode;
   const double2* c_plus;
   const double2* c_minus;
   const float2* c_plus_f;
   const float2* c_minus_f;
-  const double2* c_sd;
+  const double2* c_sd;              // n2: sum_u s_delta_u (v_ua - v_ub)^2
   const float2* c_sd_f;
   // learned terminator: predicted rho_{n+1_k} of the tier-N ADOs, row
   // (l - term_first)*K + k, used where ptr_p1 is the sentinel; null = truncation
@@ -314,6 +304,10 @@ cudaError_t launch_plus_any(int K, int n_hrchy, const int* p1, int* out, cudaStr
 cudaError_t launch_scaled_coef(int n_terms, int rows, const double2* c, double2* out, bool plus, bool sqn,
                                cudaStream_t s);
 cudaError_t launch_transpose_ados(const double2* in, double2* out, int n, long long count, cudaStream_t s);
+// `count` n x n blocks into (W^dagger X W) or out of (W X W^dagger) the basis W (row-major,
+// a column per basis vector); in_t, out_t: blocks stored column-major on that side.  Out of place.
+cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, int n, long long count, bool into,
+                          bool in_t, bool out_t, cudaStream_t s);
 cudaError_t launch_ctl_init(DpCtl* c, double t, double dt, double t_bound, double atol, double rtol, int cur,
                             cudaStream_t s);
 cudaError_t launch_ctl_set_fixed(DpCtl* c, double dt, cudaStream_t s);

@@ -2250,6 +2250,66 @@ cudaError_t launch_transpose_ados(const double2* in, double2* out, int n, long l
   return cudaGetLastError();
 }
 
+// A CTA takes `per` blocks at a time: the blocks and W in shared memory, the
+// left product beside them, the right product on the way out.  Runs twice a
+// solve, beside the copies of the state.
+__global__ void __launch_bounds__(256) k_rotate(const double2* __restrict__ in, double2* __restrict__ out,
+                                                const double2* __restrict__ W, int n, long long count, int per,
+                                                int into, int in_t, int out_t) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n2 = n * n;
+  double2* Ws = reinterpret_cast<double2*>(smem_raw);
+  double2* X = Ws + n2;
+  double2* T = X + static_cast<size_t>(per) * n2;
+  // A = W^dagger (into) or W: T = A X, out = T A^dagger
+  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+    const int a = i / n, b = i - a * n;
+    const double2 w = into ? W[b * n + a] : W[i];
+    Ws[i] = make_double2(w.x, into ? -w.y : w.y);
+  }
+  for (long long l0 = static_cast<long long>(blockIdx.x) * per; l0 < count; l0 += static_cast<long long>(gridDim.x) * per) {
+    const int ne = static_cast<int>(min(static_cast<long long>(per), count - l0)) * n2;
+    __syncthreads();
+    for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+      const int lt = i / n2, e = i - lt * n2, a = e / n, b = e - a * n;
+      X[in_t ? lt * n2 + b * n + a : i] = in[l0 * n2 + i];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+      const int lt = i / n2, e = i - lt * n2, a = e / n, b = e - a * n;
+      double2 acc = make_double2(0.0, 0.0);
+      for (int c = 0; c < n; ++c) cfma(acc, Ws[a * n + c], X[lt * n2 + c * n + b]);
+      T[i] = acc;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ne; i += blockDim.x) {
+      const int lt = i / n2, e = i - lt * n2;
+      const int a = out_t ? e % n : e / n, b = out_t ? e / n : e % n;
+      double2 acc = make_double2(0.0, 0.0);
+      for (int c = 0; c < n; ++c) {
+        const double2 w = Ws[b * n + c];
+        cfma(acc, T[lt * n2 + a * n + c], make_double2(w.x, -w.y));
+      }
+      out[l0 * n2 + i] = acc;
+    }
+  }
+}
+
+cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, int n, long long count, bool into,
+                          bool in_t, bool out_t, cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  const int n2 = n * n, per = std::max(1, 256 / n2);
+  const size_t smem = sizeof(double2) * static_cast<size_t>(n2) * (1 + 2 * per);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
+  const int grid = static_cast<int>(std::min<long long>((count + per - 1) / per, 152 * 8));
+  k_rotate<<<grid, 256, smem, s>>>(in, out, W, n, count, per, into ? 1 : 0, in_t ? 1 : 0, out_t ? 1 : 0);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
 // ------------------------------------------------------------------ arithmetic peak probe
 // Register-only FMA chains (8 independent per thread, one store per thread):
 // the FP64 and FP32 FMA rates of this GPU, the denominators of the

@@ -1231,7 +1231,7 @@ ResidentArgs resident_args(heomgb_qme_solver* qs) {
   }
   a.partials = qs->res_partials;
   a.bar = qs->res_bar;
-  a.n_total = qs->N;
+  a.root_n = std::sqrt(static_cast<double>(qs->N));
   a.max_attempts = 2000000LL;
   a.n_steps = 0;
   a.dt_step = a.dt_last = 0.0;

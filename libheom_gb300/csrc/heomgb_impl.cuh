@@ -200,7 +200,7 @@ struct ResidentArgs {
   float2* Ytmp[2];          // stage inputs 2..6 for the neighbour gathers (alternating)
   double* partials;         // per-CTA error-norm partial sums (grid entries)
   unsigned long long* bar;  // grid barrier: kResidentBarWords words, zero at launch (grid_barrier)
-  long long n_total;        // elements of the state
+  double root_n;            // square root of the state's element count (error norm)
   long long max_attempts;   // attempts before the interval gives up (status 3)
   long long n_steps;        // RK4, LSRK4: steps of dt_step before the last step of dt_last
   double dt_step, dt_last;

@@ -165,9 +165,10 @@ __device__ __forceinline__ void ff_add_prod(float& hi, float& lo, float bh, floa
 // scales the next step, FP32 resolves it far below the form's own rounding,
 // and an FP64 pow is thousands of cycles on this part's FP64 pipe, on the
 // critical path between two attempts.  The FP64 form keeps the reference's
-// FP64 pow, so its step sequence follows the reference's.
-static __device__ void dp_control(DpCtl* c, double sumsq, long long n, bool fast) {
-  const double err = sqrt(sumsq) / sqrt(static_cast<double>(n));
+// FP64 pow, so its step sequence follows the reference's.  root_n: the square
+// root of the element count.
+static __device__ void dp_control(DpCtl* c, double sumsq, double root_n, bool fast) {
+  const double err = sqrt(sumsq) / root_n;
   c->err = err;
   c->attempts += 1;
   c->count += 1;
@@ -466,7 +467,9 @@ __device__ __forceinline__ double epilogue(const Stage& st, size_t g, cx_t<TC> D
   return epi_post<TC>(st, g, Dc, dt, cur, p);
 }
 
-// Block-level sum of `v`; result valid in thread 0.
+// Block-level sum of `v`; result valid in thread 0.  The second level starts at
+// the width that the warps' sums fill (beyond it lie zeros, and an FP64 addition
+// is about 100 cycles on the way from one attempt to the next).
 __device__ __forceinline__ double block_sum(double v) {
   __shared__ double warp_part[32];
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -477,7 +480,9 @@ __device__ __forceinline__ double block_sum(double v) {
   v = 0.0;
   if (w == 0) {
     v = lane < nw ? warp_part[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    int o = 16;
+    while (o >= nw) o >>= 1;
+    for (; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   }
   __syncthreads();
   return v;
@@ -503,7 +508,7 @@ static __device__ void dp7_finish(const Stage& st, double local, long long n_tot
   v = block_sum(v);
   if (threadIdx.x == 0) {
     st.ctl->arrive = 0;
-    dp_control(st.ctl, v, n_total, st.bulk_separate != 0);
+    dp_control(st.ctl, v, sqrt(static_cast<double>(n_total)), st.bulk_separate != 0);
   }
 }
 

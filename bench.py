@@ -359,7 +359,8 @@ def secondary_aggregate24(stream, fma_peaks, steps=3):
         tune = qs.tuning()
         entry = {"value": upd / (statistics.median(ms) / 1e3), "unit": "ADO-updates/s",
                  "ms_per_solve": statistics.median(ms), "avg_stage_kernel_us": 1e6 * avg_s,
-                 "kernel": "k_rhs_sites" if tune.get("sites") else "k_rhs_diag", "tuning": tune}
+                 "kernel": "k_rhs_sites" if tune.get("sites") else "k_rhs_rows" if tune.get("rows") else "k_rhs_diag",
+                 "tuning": tune}
         if form == "mixed":
             entry["roofline"] = {"bound": "hbm", "achieved": alg / avg_s / 1e9, "peak": peak, "unit": "GB/s",
                                  "frac": alg / avg_s / 1e9 / peak, "peak_source": peak_kind,
@@ -598,7 +599,9 @@ def run_ours(args):
                   + ("" if all(t.get("local", False) for t in part_tunings) else "; k_rhs_diag for the other part"))
     else:
         kernel = ("k_rhs_sites (site-local baths: fused RHS + stage epilogue)"
-                  if any(t.get("sites", False) for t in part_tunings) else "k_rhs_diag (fused RHS + stage epilogue)")
+                  if any(t.get("sites", False) for t in part_tunings)
+                  else "k_rhs_rows (site-local baths: fused RHS + stage epilogue)"
+                  if any(t.get("rows", False) for t in part_tunings) else "k_rhs_diag (fused RHS + stage epilogue)")
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": profile_traffic(args.workload, args.form), "peak_source": peak_kind,
             "kernel": kernel,

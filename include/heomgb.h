@@ -225,6 +225,12 @@ heomgb_status heomgb_qme_solver_site_kernel(const heomgb_qme_solver* qs, int* on
  * (rk4.h:40-65) and lsrk4::solve_fixed_step (lsrk4.h:32-47) issue every
  * stage's BLAS calls from the host. */
 heomgb_status heomgb_qme_solver_resident(const heomgb_qme_solver* qs, int* on, int* grid, int* ados_per_cta);
+/* 1 when the solver's stages run the row kernel (site-local baths of at most 32
+ * levels in the mixed form, models and batches; heomgb_qme_solver_tuning's
+ * elems_per_thread is then the ADOs that a warp takes).  It joins the search
+ * where every instance is eligible; HEOMGB_ROWS=0 keeps it out, =1 takes it
+ * before k_rhs_diag.  No reference counterpart. */
+heomgb_status heomgb_qme_solver_row_kernel(const heomgb_qme_solver* qs, int* on);
 /* Whether fixed steps run as cluster-resident intervals (one launch per output
  * interval, a thread-block cluster of `size` CTAs of `block` threads per bin of
  * instances).  No reference counterpart. */

@@ -231,6 +231,7 @@ struct DiagPlan {
   int block = 128, ept = 4, grid = 1, min_blocks = 1;
   bool tcore = false;  // commutators on the tensor cores (k_rhs_diag_tc)
   bool sites = false;  // the site-local-bath kernel (k_rhs_sites)
+  bool rows = false;   // the row kernel (k_rhs_rows)
 };
 
 // Whether an instance can take the tensor-core commutator: mixed form, a
@@ -299,7 +300,9 @@ void build_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int block, int 
   P.ds.sites_hreal = (sites_tile > 0 && P.inst[0].h_real) ? 1 : 0;
   P.ds.sites_minb = sites_tile > 0 ? min_blocks : 0;
   P.ds.sites_rt = sites_tile > 0 ? sites_rt : 0;
+  P.ds.rows = 0;
   P.sites = sites_tile > 0;
+  P.rows = false;
   P.tcore = tcore;
   P.block = block;
   P.ept = ept;
@@ -310,6 +313,54 @@ void build_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int block, int 
   const long long per_sm = sites_tile > 0 ? min_blocks : 2048 / block;
   P.grid = static_cast<int>(std::max<long long>(
       1, std::min<long long>(static_cast<long long>(tiles.size()), static_cast<long long>(n_sm) * per_sm)));
+  ck(cudaStreamSynchronize(s), "plan upload");
+}
+
+// The row kernel's plan (k_rhs_rows, for the epilogues of stage kind `kind`):
+// warps that take `ados` ADOs at a time.  One resident wave of CTAs, divided
+// among the instances by their ADOs (at least one each; a CTA beyond the wave
+// follows another); a CTA takes every c-th group of its instance's c CTAs, so
+// each gets its share of the low tiers, whose ADOs have +1 terms.
+void build_rows_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int block, int ados, int kind, int n_sm,
+                     cudaStream_t s) {
+  P.arena.release();
+  P.inst = insts;
+  DiagSet& ds = P.ds;
+  ds = DiagSet{};
+  ds.rows = 1;
+  ds.min_blocks = 1;
+  ds.rows_n = insts[0].n <= 8 ? insts[0].n : 0;
+  long long all = 0;
+  for (DiagInst& I : P.inst) {
+    if (!rows_eligible(I, true)) throw unsupported_error("row kernel: instance not eligible");
+    if (I.n != insts[0].n) ds.rows_n = 0;
+    I.tile = ados;
+    ds.rows_tab = std::max(ds.rows_tab, rows_tables(I));
+    ds.rows_warp = std::max(ds.rows_warp, rows_warp(I, ados));
+    ds.total = std::max(ds.total, I.elem_off + static_cast<long long>(I.n2) * I.nh);
+    all += I.nh;
+  }
+  if (ds.rows_n > 0 && ados * ds.rows_n > 32) throw unsupported_error("row kernel: more rows than lanes");
+  const int warps = block / 32;
+  ds.smem = ds.rows_tab + warps * ds.rows_warp;
+  const int per_sm = ds.smem <= 200 * 1024 ? rows_resident(ds, kind, block) : 0;
+  if (per_sm < 1) throw unsupported_error("row kernel: the groups do not fit an SM");
+  const long long wave = static_cast<long long>(n_sm) * per_sm;
+  std::vector<DiagTile> tiles;
+  for (size_t i = 0; i < P.inst.size(); ++i) {
+    const long long nh = P.inst[i].nh, groups = (nh + ados - 1) / ados;
+    const int c = static_cast<int>(std::max<long long>(1, std::min(wave * nh / std::max(1ll, all), (groups + warps - 1) / warps)));
+    for (int j = 0; j < c; ++j) tiles.push_back(DiagTile{static_cast<int>(i), j, c, 0});
+  }
+  ds.inst = P.arena.upload(P.inst, s);
+  ds.tiles = P.arena.upload(tiles, s);
+  ds.n_tiles = static_cast<int>(tiles.size());
+  P.sites = P.tcore = false;
+  P.rows = true;
+  P.block = block;
+  P.ept = ados;
+  P.min_blocks = 1;
+  P.grid = static_cast<int>(std::min<long long>(ds.n_tiles, wave));
   ck(cudaStreamSynchronize(s), "plan upload");
 }
 
@@ -789,6 +840,11 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
       int4* rec = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
       di.site_rec = rec;
       ck(launch_site_records(di, dms, rec, s), "site records");
+      if (rows_eligible(di, q->precision_eff == HEOMGB_MIXED)) {
+        int4* rr = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
+        ck(launch_rows_records(di, rr, s), "row records");
+        di.rows_rec = rr;
+      }
       ck(cudaStreamSynchronize(s), "site records sync");
     }
   }
@@ -1483,13 +1539,44 @@ void autotune(heomgb_qme_solver* qs) {
       }
   }
   if (pin_sb && !best_sites) throw unsupported_error("HEOMGB_TILE=sites: the pinned shape does not fit");
+  // the row kernel joins where every instance is eligible and the stage input is
+  // the FP32 copy (16 instances of 7 sites, depth 4: 48 us a stage, k_rhs_diag 74;
+  // a single one is 12 against 9: its warps get one group each, and a group is a
+  // long chain); HEOMGB_ROWS=0 keeps it out, =1 keeps k_rhs_diag out
+  bool rows_ok = qs->separate, rows_only = false, best_rows = false;
+  for (const DiagInst& I : insts) rows_ok = rows_ok && rows_eligible(I, qs->mixed);
+  if (const char* env = std::getenv("HEOMGB_ROWS")) {
+    if (std::string(env) == "0") rows_ok = false;
+    rows_only = rows_ok && std::string(env) == "1";
+  }
+  if (rows_ok && !pin_tc && !pin_sb && !pin_b) {
+    std::vector<int> groups = {std::max(1, 32 / insts[0].n)};
+    while (groups.back() > 1) groups.push_back(groups.back() / 2);
+    for (int b : {64, 128, 256})
+      for (int e : groups) {
+        try {
+          build_rows_plan(qs->plan, insts, b, e, st.kind, q->n_sm, qs->stream);
+        } catch (const unsupported_error&) {
+          continue;
+        }
+        const float ms = time_plan(b);
+        log_shape("rows (x = ADOs per warp)", b, e, 1, ms);
+        if (ms < best) {
+          best = ms;
+          best_b = b;
+          best_e = e;
+          best_tc = best_sites = false;
+          best_rows = true;
+        }
+      }
+  }
   const int blocks[3] = {64, 128, 256}, epts[4] = {1, 2, 4, 8};
   const int n_minb = qs->mixed ? 3 : 1, minbs[3] = {1, 3, 4};
   for (int b : blocks)
     for (int e : epts)
       for (int mi = 0; mi < n_minb; ++mi) {
       const int m = minbs[mi];
-      if (pin_tc || pin_sb || (pin_b && (b != pin_b || e != pin_e || m != pin_m))) continue;
+      if (pin_tc || pin_sb || (rows_only && best_rows) || (pin_b && (b != pin_b || e != pin_e || m != pin_m))) continue;
       try {
         build_plan(qs->plan, insts, b, e, m, qs->mixed, q->n_sm, qs->stream);
       } catch (const unsupported_error&) {
@@ -1508,14 +1595,15 @@ void autotune(heomgb_qme_solver* qs) {
         best_b = b;
         best_e = e;
         best_m = m;
-        best_tc = false;
-        best_sites = false;
+        best_tc = best_sites = best_rows = false;
       }
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   qs->stage_ms = best < 1e29f ? best / 3.f : 0.f;
-  if (best_sites)
+  if (best_rows)
+    build_rows_plan(qs->plan, insts, best_b, best_e, st.kind, q->n_sm, qs->stream);
+  else if (best_sites)
     build_plan(qs->plan, insts, best_sb, 1, best_sm, qs->mixed, q->n_sm, qs->stream, false, best_st, best_sr);
   else if (best_tc)
     build_plan(qs->plan, insts, best_tc_b, 1, best_tc_m, qs->mixed, q->n_sm, qs->stream, true);
@@ -2759,6 +2847,13 @@ heomgb_status heomgb_qme_solver_resident(const heomgb_qme_solver* qs, int* on, i
     *on = qs->resident ? 1 : 0;
     if (grid) *grid = qs->resident ? qs->res_grid : 0;
     if (ados_per_cta) *ados_per_cta = qs->resident ? qs->res_apc : 0;
+  });
+}
+
+heomgb_status heomgb_qme_solver_row_kernel(const heomgb_qme_solver* qs, int* on) {
+  return guard([&] {
+    require(qs != nullptr && on != nullptr, "null argument");
+    *on = qs->path == PATH_DIAG && qs->plan.rows ? 1 : 0;
   });
 }
 

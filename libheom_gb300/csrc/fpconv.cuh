@@ -72,9 +72,10 @@ HEOMGB_HD int fc_msb(uint32_t v) {
 #define HEOMGB_COLD static inline
 #endif
 
-// float -> double (exact).  The common case (a normal float) is a few integer
-// operations; zeros, subnormals, infinities and NaNs take a separate call so
-// that the compiler does not predicate their paths into every conversion.
+// float -> double (exact).  The common cases (a normal float, and a zero:
+// ADOs that the dynamics has not reached yet) are a few integer operations;
+// subnormals, infinities and NaNs take a separate call so that the compiler
+// does not predicate their paths into every conversion.
 HEOMGB_COLD uint64_t f2d_rare(uint32_t u) {
   const uint64_t sign = static_cast<uint64_t>(u >> 31) << 63;
   const uint32_t ex = (u >> 23) & 0xffu, man = u & 0x7fffffu;
@@ -86,9 +87,11 @@ HEOMGB_COLD uint64_t f2d_rare(uint32_t u) {
 HEOMGB_HD double f2d(float x) {
   const uint32_t u = fc_f2u(x);
   const uint32_t ex = (u >> 23) & 0xffu;
-  if (ex - 1u < 0xfeu)  // normal: rebias the exponent (1023 - 127), widen the fraction
-    return fc_u2d((static_cast<uint64_t>(u >> 31) << 63) | (static_cast<uint64_t>(ex + 896u) << 52) |
-                  (static_cast<uint64_t>(u & 0x7fffffu) << 29));
+  const bool zero = (u << 1) == 0u;
+  if (ex - 1u < 0xfeu || zero) {  // normal: rebias the exponent (1023 - 127), widen the fraction
+    const uint32_t hi = (u & 0x80000000u) | (zero ? 0u : ((u & 0x7fffffffu) >> 3) + (896u << 20));
+    return fc_u2d((static_cast<uint64_t>(hi) << 32) | (u << 29));
+  }
   return fc_u2d(f2d_rare(u));
 }
 

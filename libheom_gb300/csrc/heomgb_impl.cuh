@@ -160,6 +160,7 @@ struct DiagInst {
   int site_w;               // entries per ADO (max(1, min(K, max_depth)))
   const int4* site_rec;     // nh * (1 + site_w)
   const float2* site_cm3;   // K * 3
+  const int4* rows_rec;     // nh * (1 + site_w): the records as k_rhs_rows reads them (instances that it takes)
   const float2* site_cp2;   // K * 2: the +1 coefficient of mode k in its site's row / column
   const int* site_ptr;      // n + 1: the modes of site s are site_modes[site_ptr[s] .. site_ptr[s+1])
   const int* site_modes;    // K, per site in increasing k
@@ -183,6 +184,10 @@ struct DiagSet {
   int sites_hreal;          // its instance has a real H
   int sites_minb;           // its resident CTAs per SM (2, 3 or 4)
   int sites_rt;             // its rows per register block (4 or 2)
+  int rows;                 // 1: the row kernel (k_rhs_rows; mixed form, every instance eligible)
+  int rows_n;               // its levels where all instances share 2..8 of them, else 0
+  size_t rows_tab;          // its shared memory: the instance's tables, then a part per warp
+  size_t rows_warp;
 };
 
 // Resident intervals (k_dp_resident: Dormand-Prince; k_rk4_resident and
@@ -292,6 +297,14 @@ bool sites_eligible(const DiagInst& I, bool mixed);
 size_t sites_smem(int n, int K, int tile, int w);
 bool sites_variant(int rows, int min_blocks, int block);  // a compiled (rows, CTAs per SM, CTA size) variant
 cudaError_t launch_site_records(const DiagInst& I, const int* msite, int4* rec, cudaStream_t s);
+cudaError_t launch_rows(const DiagSet& ds, const Stage& st, int grid, int block, cudaStream_t s);
+// rows.cu: whether an instance can take k_rhs_rows, the bytes of its tables and of a warp that takes `ados` ADOs at a
+// time, the resident CTAs per SM for a stage epilogue
+bool rows_eligible(const DiagInst& I, bool mixed);
+cudaError_t launch_rows_records(const DiagInst& I, int4* rec, cudaStream_t s);
+size_t rows_tables(const DiagInst& I);
+size_t rows_warp(const DiagInst& I, int ados);
+int rows_resident(const DiagSet& ds, int kind, int block);
 cudaError_t launch_sites(const DiagSet& ds, const Stage& st, int grid, int block, cudaStream_t s);
 
 cudaError_t launch_hrchy_build(int K, int depth, int n_hrchy, const long long* binom, int binom_dim, int* nidx,

@@ -57,14 +57,6 @@ __host__ __device__ inline size_t tc_operand_bytes(int n) {
 __host__ __device__ inline size_t tc_product_bytes(int n, int tile) {
   return 4 * sizeof(float) * static_cast<size_t>(tile) * n * (n + 1) + sizeof(float2) * static_cast<size_t>(tile) * n * n;
 }
-// x / d for 0 <= x < 2^16 and 1 <= d <= 2^12 from rd = 1.0f / d (correctly
-// rounded): (x + 0.5) / d lies at least 0.5 / d away from an integer and the
-// two roundings move it by less than (x / d + 1) * 2^-23, so truncation gives
-// the exact quotient (checked exhaustively over that range against integer
-// division)
-__device__ __forceinline__ int small_div(int x, float rd) {
-  return __float2int_rz(__fmul_rn(static_cast<float>(x) + 0.5f, rd));
-}
 __host__ __device__ inline size_t tc_b_bytes(int n) {
   const TcGeom t = tc_geom(n);
   return 2 * sizeof(float) * (static_cast<size_t>(t.n_pad) * t.k_pad);
@@ -2041,7 +2033,10 @@ static cudaError_t launch_typed(const RhsModel& m, const DiagSet* ds, const Stag
   const size_t smem = rhs_smem_bytes(m, path, std::is_same<TC, float>::value);
   if (path == PATH_DIAG) {
     if constexpr (std::is_same<TC, float>::value && std::is_same<TB, float2>::value)
-      if (ds->sites) return launch_sites(*ds, st, grid, block, s);  // counts its own launch
+    {  // these count their own launch
+      if (ds->rows) return launch_rows(*ds, st, grid, block, s);
+      if (ds->sites) return launch_sites(*ds, st, grid, block, s);
+    }
     const size_t dsm = ds->smem;
     // the register-capped variant exists for the FP32 arithmetic only (the
     // FP64 kernel would spill at 80 registers)

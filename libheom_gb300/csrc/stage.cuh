@@ -159,6 +159,15 @@ __device__ __forceinline__ void ff_add_prod(float& hi, float& lo, float bh, floa
   lo = __fadd_rn(lo, __fadd_rn(__fadd_rn(err, pe), __fmul_rn(bl, k)));
 }
 
+// x / d for 0 <= x < 2^16 and 1 <= d <= 2^12 from rd = 1.0f / d (correctly
+// rounded): (x + 0.5) / d lies at least 0.5 / d away from an integer and the
+// two roundings move it by less than (x / d + 1) * 2^-23, so truncation gives
+// the exact quotient (checked exhaustively over that range against integer
+// division)
+__device__ __forceinline__ int small_div(int x, float rd) {
+  return __float2int_rz(__fmul_rn(static_cast<float>(x) + 0.5f, rd));
+}
+
 // ------------------------------------------------------------------ step control
 // rkdp.h:150-177 and adaptive_step_size_solver.h:45-55, one thread.  The
 // mixed form takes the step-size factor err^-0.2 in FP32 (`fast`): it only

@@ -232,6 +232,7 @@ struct DiagPlan {
   bool tcore = false;  // commutators on the tensor cores (k_rhs_diag_tc)
   bool sites = false;  // the site-local-bath kernel (k_rhs_sites)
   bool rows = false;   // the row kernel (k_rhs_rows)
+  bool split = false;  // the FP64 stages with the commutator on the tensor cores (k_rhs_split)
 };
 
 // Whether an instance can take the tensor-core commutator: mixed form, a
@@ -300,7 +301,8 @@ void build_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int block, int 
   P.ds.sites_hreal = (sites_tile > 0 && P.inst[0].h_real) ? 1 : 0;
   P.ds.sites_minb = sites_tile > 0 ? min_blocks : 0;
   P.ds.sites_rt = sites_tile > 0 ? sites_rt : 0;
-  P.ds.rows = 0;
+  P.ds.rows = P.ds.split = 0;
+  P.split = false;
   P.sites = sites_tile > 0;
   P.rows = false;
   P.tcore = tcore;
@@ -313,6 +315,46 @@ void build_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int block, int 
   const long long per_sm = sites_tile > 0 ? min_blocks : 2048 / block;
   P.grid = static_cast<int>(std::max<long long>(
       1, std::min<long long>(static_cast<long long>(tiles.size()), static_cast<long long>(n_sm) * per_sm)));
+  ck(cudaStreamSynchronize(s), "plan upload");
+}
+
+// The FP64 stages with the commutator on the tensor cores (k_rhs_split): two
+// resident CTAs per SM (their tensor memory and shared memory).
+void build_split_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int n_sm, cudaStream_t s) {
+  P.arena.release();
+  P.inst = insts;
+  DiagSet& ds = P.ds;
+  ds = DiagSet{};
+  ds.split = 1;
+  ds.min_blocks = 1;
+  std::vector<DiagTile> tiles;
+  size_t ma = 0, mb = 0, my = 0;
+  for (size_t i = 0; i < P.inst.size(); ++i) {
+    DiagInst& I = P.inst[i];
+    if (!split_eligible(I, false)) throw unsupported_error("split commutator: instance not eligible");
+    size_t a, b, y;
+    split_smem(I, &a, &b, &y);
+    ma = std::max(ma, a);
+    mb = std::max(mb, b);
+    my = std::max(my, y);
+    I.tile = split_tile(I.n);
+    for (int l0 = 0; l0 < I.nh; l0 += I.tile)
+      tiles.push_back(DiagTile{static_cast<int>(i), l0, std::min(I.tile, I.nh - l0), 0});
+    ds.total = std::max(ds.total, I.elem_off + static_cast<long long>(I.n2) * I.nh);
+  }
+  ds.split_b = ma;
+  ds.split_y = ma + mb;
+  ds.smem = ma + mb + my;
+  if (ds.smem > 200 * 1024) throw unsupported_error("split commutator: tile exceeds shared memory");
+  ds.inst = P.arena.upload(P.inst, s);
+  ds.tiles = P.arena.upload(tiles, s);
+  ds.n_tiles = static_cast<int>(tiles.size());
+  P.sites = P.rows = P.tcore = false;
+  P.split = true;
+  P.block = split_threads();
+  P.ept = 1;
+  P.min_blocks = 1;
+  P.grid = std::max(1, std::min(ds.n_tiles, 2 * n_sm));
   ck(cudaStreamSynchronize(s), "plan upload");
 }
 
@@ -355,7 +397,7 @@ void build_rows_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int block,
   ds.inst = P.arena.upload(P.inst, s);
   ds.tiles = P.arena.upload(tiles, s);
   ds.n_tiles = static_cast<int>(tiles.size());
-  P.sites = P.tcore = false;
+  P.sites = P.tcore = P.split = false;
   P.rows = true;
   P.block = block;
   P.ept = ados;
@@ -840,6 +882,12 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
       int4* rec = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
       di.site_rec = rec;
       ck(launch_site_records(di, dms, rec, s), "site records");
+      if (q->precision_eff == HEOMGB_FP64 && di.h_sym && n >= 4 && n <= 32) {
+        std::vector<double> Hr(n2);
+        for (int e = 0; e < n2; ++e) Hr[e] = H[e].real();
+        const std::vector<unsigned short> dig = split_h_digits(Hr.data(), n, &di.h_exp);
+        if (!dig.empty()) di.h_digits = reinterpret_cast<const uint4*>(q->arena.upload(dig, s));
+      }
       if (rows_eligible(di, q->precision_eff == HEOMGB_MIXED)) {
         int4* rr = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
         ck(launch_rows_records(di, rr, s), "row records");
@@ -1570,13 +1618,38 @@ void autotune(heomgb_qme_solver* qs) {
         }
       }
   }
+  // FP64: the commutator on the tensor cores where every instance is eligible;
+  // HEOMGB_SPLIT=0 keeps it out, =1 keeps k_rhs_diag out
+  bool split_ok = !insts.empty(), split_only = false, best_split = false;
+  for (const DiagInst& I : insts) split_ok = split_ok && split_eligible(I, qs->mixed);
+  if (const char* env = std::getenv("HEOMGB_SPLIT")) {
+    if (std::string(env) == "0") split_ok = false;
+    split_only = split_ok && std::string(env) == "1";
+  }
+  if (split_ok && !pin_b) {
+    try {
+      build_split_plan(qs->plan, insts, q->n_sm, qs->stream);
+      const float ms = time_plan(split_threads());
+      log_shape("split", split_threads(), 1, 1, ms);
+      DpCtl probe;
+      ck(cudaMemcpyAsync(&probe, qs->ctl, sizeof(DpCtl), cudaMemcpyDeviceToHost, qs->stream), "ctl read");
+      ck(cudaStreamSynchronize(qs->stream), "ctl sync");
+      if (probe.status == 2) {
+        ck(cudaMemsetAsync(&qs->ctl->status, 0, sizeof(int), qs->stream), "ctl reset");
+      } else if (ms < best) {
+        best = ms;
+        best_split = true;
+      }
+    } catch (const unsupported_error&) {
+    }
+  }
   const int blocks[3] = {64, 128, 256}, epts[4] = {1, 2, 4, 8};
   const int n_minb = qs->mixed ? 3 : 1, minbs[3] = {1, 3, 4};
   for (int b : blocks)
     for (int e : epts)
       for (int mi = 0; mi < n_minb; ++mi) {
       const int m = minbs[mi];
-      if (pin_tc || pin_sb || (rows_only && best_rows) || (pin_b && (b != pin_b || e != pin_e || m != pin_m))) continue;
+      if (pin_tc || pin_sb || (rows_only && best_rows) || (split_only && best_split) || (pin_b && (b != pin_b || e != pin_e || m != pin_m))) continue;
       try {
         build_plan(qs->plan, insts, b, e, m, qs->mixed, q->n_sm, qs->stream);
       } catch (const unsupported_error&) {
@@ -1595,13 +1668,15 @@ void autotune(heomgb_qme_solver* qs) {
         best_b = b;
         best_e = e;
         best_m = m;
-        best_tc = best_sites = best_rows = false;
+        best_tc = best_sites = best_rows = best_split = false;
       }
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   qs->stage_ms = best < 1e29f ? best / 3.f : 0.f;
-  if (best_rows)
+  if (best_split)
+    build_split_plan(qs->plan, insts, q->n_sm, qs->stream);
+  else if (best_rows)
     build_rows_plan(qs->plan, insts, best_b, best_e, st.kind, q->n_sm, qs->stream);
   else if (best_sites)
     build_plan(qs->plan, insts, best_sb, 1, best_sm, qs->mixed, q->n_sm, qs->stream, false, best_st, best_sr);
@@ -1738,7 +1813,8 @@ void plan_local(heomgb_qme_solver* qs) {
   const NvtxRange range("heomgb plan: instance-resident bins");
   heomgb_qme* q = qs->q;
   qs->local = false;
-  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || qs->path != PATH_DIAG || qs->term || qs->plan.tcore)
+  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || qs->path != PATH_DIAG || qs->term || qs->plan.tcore ||
+      qs->plan.split)
     return;
   const int scheme = resident_scheme(qs);
   if (qs->resident && qs->res_step_ms <= 0.f) return;  // an untimed (pinned) resident plan stays
@@ -2271,7 +2347,7 @@ void solve_fixed(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwarg
   ck(launch_ctl_set_fixed(qs->ctl, last, qs->stream), "ctl dt");
   replay(qs, false);
   busy_end(qs);
-  if (qs->plan.tcore) {  // a tensor-core stage that gave up flags the controller
+  if (qs->plan.tcore || qs->plan.split) {  // a tensor-core stage that gave up flags the controller
     ck(cudaMemcpyAsync(qs->ctl_host, qs->ctl, sizeof(DpCtl), cudaMemcpyDeviceToHost, qs->stream), "ctl read");
     ck(cudaStreamSynchronize(qs->stream), "ctl sync");
     if (qs->ctl_host->status == 2) throw cuda_error("tensor-core stage did not complete");
@@ -2854,6 +2930,13 @@ heomgb_status heomgb_qme_solver_row_kernel(const heomgb_qme_solver* qs, int* on)
   return guard([&] {
     require(qs != nullptr && on != nullptr, "null argument");
     *on = qs->path == PATH_DIAG && qs->plan.rows ? 1 : 0;
+  });
+}
+
+heomgb_status heomgb_qme_solver_split(const heomgb_qme_solver* qs, int* on) {
+  return guard([&] {
+    require(qs != nullptr && on != nullptr, "null argument");
+    *on = qs->path == PATH_DIAG && qs->plan.split ? 1 : 0;
   });
 }
 

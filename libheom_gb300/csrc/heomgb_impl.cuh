@@ -7,6 +7,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 struct heomgb_mlp;
 
@@ -166,6 +167,9 @@ struct DiagInst {
   const int* site_modes;    // K, per site in increasing k
   const double2* site_cm3_d;  // K * 3 and K * 2: the same coefficients in FP64 (the FP64 resident interval)
   const double2* site_cp2_d;
+  // k_rhs_split (FP64, real symmetric H): H's digits as its B operand, and the exponent of their scale
+  const uint4* h_digits;
+  int h_exp;
 };
 struct DiagTile {
   int inst, l0, nt, pad;
@@ -188,6 +192,8 @@ struct DiagSet {
   int rows_n;               // its levels where all instances share 2..8 of them, else 0
   size_t rows_tab;          // its shared memory: the instance's tables, then a part per warp
   size_t rows_warp;
+  int split;                // 1: the FP64 stage with the commutator on the tensor cores (k_rhs_split)
+  size_t split_b, split_y;  // its shared memory: A operand and products, B operand, stage input
 };
 
 // Resident intervals (k_dp_resident: Dormand-Prince; k_rk4_resident and
@@ -297,6 +303,14 @@ bool sites_eligible(const DiagInst& I, bool mixed);
 size_t sites_smem(int n, int K, int tile, int w);
 bool sites_variant(int rows, int min_blocks, int block);  // a compiled (rows, CTAs per SM, CTA size) variant
 cudaError_t launch_site_records(const DiagInst& I, const int* msite, int4* rec, cudaStream_t s);
+// split.cu: H (n x n, row-major, real) as the digits of k_rhs_split's B operand (empty: out of range), whether an
+// instance can take the kernel, its ADOs per tile, threads and shared memory
+std::vector<unsigned short> split_h_digits(const double* H, int n, int* exponent);
+bool split_eligible(const DiagInst& I, bool mixed);
+int split_tile(int n);
+int split_threads();
+void split_smem(const DiagInst& I, size_t* a, size_t* b, size_t* y);
+cudaError_t launch_split(const DiagSet& ds, const Stage& st, int grid, cudaStream_t s);
 cudaError_t launch_rows(const DiagSet& ds, const Stage& st, int grid, int block, cudaStream_t s);
 // rows.cu: whether an instance can take k_rhs_rows, the bytes of its tables and of a warp that takes `ados` ADOs at a
 // time, the resident CTAs per SM for a stage epilogue

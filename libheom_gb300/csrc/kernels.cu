@@ -2032,6 +2032,8 @@ static cudaError_t launch_typed(const RhsModel& m, const DiagSet* ds, const Stag
                                 cudaStream_t s) {
   const size_t smem = rhs_smem_bytes(m, path, std::is_same<TC, float>::value);
   if (path == PATH_DIAG) {
+    if constexpr (std::is_same<TC, double>::value)
+      if (ds->split) return launch_split(*ds, st, grid, s);  // counts its own launch
     if constexpr (std::is_same<TC, float>::value && std::is_same<TB, float2>::value)
     {  // these count their own launch
       if (ds->rows) return launch_rows(*ds, st, grid, block, s);

@@ -333,12 +333,14 @@ class qme_solver:
         check(self._lib.heomgb_qme_solver_site_kernel(self._h, ctypes.byref(si), ctypes.byref(st)))
         ro = ctypes.c_int()
         check(self._lib.heomgb_qme_solver_row_kernel(self._h, ctypes.byref(ro)))
+        sp = ctypes.c_int()
+        check(self._lib.heomgb_qme_solver_split(self._h, ctypes.byref(sp)))
         co, cz, cn, cb = ctypes.c_int(), ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check(self._lib.heomgb_qme_solver_cluster(self._h, ctypes.byref(co), ctypes.byref(cz), ctypes.byref(cn),
                                                   ctypes.byref(cb)))
         out = dict(block=b.value, elems_per_thread=e.value, n_tiles=t.value, min_blocks=m.value,
                    tensor_cores=bool(tc.value), resident=bool(rs.value), local=bool(lo.value),
-                   sites=bool(si.value), rows=bool(ro.value), cluster=bool(co.value))
+                   sites=bool(si.value), rows=bool(ro.value), split=bool(sp.value), cluster=bool(co.value))
         if si.value:
             out.update(sites_ados_per_tile=st.value)
         if rs.value:

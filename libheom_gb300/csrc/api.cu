@@ -328,12 +328,13 @@ void build_split_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int n_sm,
   ds.split = 1;
   ds.min_blocks = 1;
   std::vector<DiagTile> tiles;
-  size_t ma = 0, mb = 0, my = 0;
+  size_t ma = 0, mp = 0, mb = 0, my = 0;
   for (size_t i = 0; i < P.inst.size(); ++i) {
     DiagInst& I = P.inst[i];
     if (!split_eligible(I, false)) throw unsupported_error("split commutator: instance not eligible");
-    size_t a, b, y;
-    split_smem(I, &a, &b, &y);
+    size_t a, p, b, y;
+    split_smem(I, &a, &p, &b, &y);
+    mp = std::max(mp, p);
     ma = std::max(ma, a);
     mb = std::max(mb, b);
     my = std::max(my, y);
@@ -342,9 +343,11 @@ void build_split_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int n_sm,
       tiles.push_back(DiagTile{static_cast<int>(i), l0, std::min(I.tile, I.nh - l0), 0});
     ds.total = std::max(ds.total, I.elem_off + static_cast<long long>(I.n2) * I.nh);
   }
-  ds.split_b = ma;
-  ds.split_y = ma + mb;
-  ds.smem = ma + mb + my;
+  ds.split_p = ma;
+  ds.split_b = ma + mp;
+  ds.split_y = ds.split_b + mb;
+  ds.split_ybuf = my;
+  ds.smem = ds.split_y + 3 * my;
   if (ds.smem > 200 * 1024) throw unsupported_error("split commutator: tile exceeds shared memory");
   ds.inst = P.arena.upload(P.inst, s);
   ds.tiles = P.arena.upload(tiles, s);
@@ -354,7 +357,8 @@ void build_split_plan(DiagPlan& P, const std::vector<DiagInst>& insts, int n_sm,
   P.block = split_threads();
   P.ept = 1;
   P.min_blocks = 1;
-  P.grid = std::max(1, std::min(ds.n_tiles, 2 * n_sm));
+  const int per_sm = ds.smem <= 112 * 1024 ? 2 : 1;
+  P.grid = std::max(1, std::min(ds.n_tiles, per_sm * n_sm));
   ck(cudaStreamSynchronize(s), "plan upload");
 }
 
@@ -887,6 +891,13 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
         for (int e = 0; e < n2; ++e) Hr[e] = H[e].real();
         const std::vector<unsigned short> dig = split_h_digits(Hr.data(), n, &di.h_exp);
         if (!dig.empty()) di.h_digits = reinterpret_cast<const uint4*>(q->arena.upload(dig, s));
+        std::vector<cd> cmn(cm3.size() * di.occ_rows);
+        for (size_t p = 0; p < cm3.size(); ++p)
+          for (int o = 0; o < di.occ_rows; ++o) {
+            const double f = di.sqrt_norm ? std::sqrt(static_cast<double>(o)) : static_cast<double>(o);
+            cmn[p * di.occ_rows + o] = cd(f * cm3[p].real(), f * cm3[p].imag());
+          }
+        di.site_cmn_d = q->arena.upload(to_d2(cmn), s);
       }
       if (rows_eligible(di, q->precision_eff == HEOMGB_MIXED)) {
         int4* rr = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));

@@ -167,6 +167,7 @@ struct DiagInst {
   const int* site_modes;    // K, per site in increasing k
   const double2* site_cm3_d;  // K * 3 and K * 2: the same coefficients in FP64 (the FP64 resident interval)
   const double2* site_cp2_d;
+  const double2* site_cmn_d;  // site_cm3_d scaled by the occupation: row (3 k + case) * occ_rows + n_k
   // k_rhs_split (FP64, real symmetric H): H's digits as its B operand, and the exponent of their scale
   const uint4* h_digits;
   int h_exp;
@@ -193,7 +194,7 @@ struct DiagSet {
   size_t rows_tab;          // its shared memory: the instance's tables, then a part per warp
   size_t rows_warp;
   int split;                // 1: the FP64 stage with the commutator on the tensor cores (k_rhs_split)
-  size_t split_b, split_y;  // its shared memory: A operand and products, B operand, stage input
+  size_t split_p, split_b, split_y, split_ybuf;  // its shared memory: A operand, products, B operand, three stage inputs
 };
 
 // Resident intervals (k_dp_resident: Dormand-Prince; k_rk4_resident and
@@ -309,7 +310,7 @@ std::vector<unsigned short> split_h_digits(const double* H, int n, int* exponent
 bool split_eligible(const DiagInst& I, bool mixed);
 int split_tile(int n);
 int split_threads();
-void split_smem(const DiagInst& I, size_t* a, size_t* b, size_t* y);
+void split_smem(const DiagInst& I, size_t* a, size_t* p, size_t* b, size_t* y);
 cudaError_t launch_split(const DiagSet& ds, const Stage& st, int grid, cudaStream_t s);
 cudaError_t launch_rows(const DiagSet& ds, const Stage& st, int grid, int block, cudaStream_t s);
 // rows.cu: whether an instance can take k_rhs_rows, the bytes of its tables and of a warp that takes `ados` ADOs at a

@@ -16,23 +16,36 @@
 // products of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012).
 // Measured on the 24-site aggregate at depth 3: a state's error against
 // extended precision is 7.0e-17 after 4 steps, 7.6e-17 with the FP64 sums; a
-// stage of 12M elements takes 1.22 ms, 2.95 with k_rhs_diag<double>, whose FP64
-// pipe alone needs 2.58.
+// stage of 12M elements takes 0.59 ms, 2.95 with k_rhs_diag<double>, whose FP64
+// pipe alone needs 2.58 (16 sites, depth 3: 0.088 and 0.287).
 //
-// Per tile of T = 128 / (4 n) ADOs:
-//   1. the stage input to shared memory, each ADO's largest exponent;
+// Per tile of T = 128 / (4 n) ADOs, the first group of a CTA (128 threads):
+//   1. the stage input (copied with cp.async a tile ahead), each ADO's largest
+//      exponent;
 //   2. digits of R, I, R^T and I^T (rho = R + iI; rows 4 n per ADO, K = n
 //      padded to 16) into the A operand, K-major without swizzle;
 //   3. MMAs (M = 128, one thread): digit i of rho against the digits 0..6-i of
 //      H at once (N = 7 - i blocks of n padded to 16), into the tensor-memory
 //      columns of the orders i..6, so 7 MMAs per 16 of K cover all 28 pairs;
 //   4. read-back: rows of R H, I H (rho H) and R^T H, I^T H (H rho,
-//      transposed) as 128-bit integers in shared memory, over the A operand;
-//   5. one element per thread: the difference of the two products in integers,
-//      one rounding to FP64 (three FP64 additions per component), damping,
-//      bath terms, stage epilogue.
-// An ADO with elements beyond 2^900, infinities or NaNs takes FP64 sums in
-// pass 5.  Two CTAs per SM overlap each other's passes.
+//      transposed) as 64-bit integers (60 bits of each product) in shared memory;
+// and the second group (320 threads), a tile behind it:
+//   5. one element per thread: the difference of the two products, rounded to
+//      FP64 with integer operations; damping and +1 terms (ADOs below the
+//      deepest tier);
+//   6. the -1 terms, one thread per element that a mode touches (an FP64
+//      instruction takes the pipe's 64 cycles whatever lanes it has: inside
+//      pass 5 these terms' few lanes made every warp pay, 0.44 of 1.22 ms);
+//   7. the stage epilogue, one element per thread.
+// The groups meet on named barriers: products full (first to second) and free
+// (second to first).  Two CTAs per SM, by tensor memory (256 of 512 columns)
+// and registers.  What bounds it now is the second group's chain: FP64 issue
+// (0.35 ms of the 0.59 a stage of 12M elements takes) and shared memory
+// latency; the first group alone takes 0.38.  Measured there: one group with
+// CTA barriers between the passes 0.86 ms; groups of 256 and 192 threads 0.69;
+// conversions and scaling on the FP64 pipe 0.69, the epilogue's loads ahead of
+// pass 5 0.63 (registers).  An ADO with elements beyond 2^900, infinities or
+// NaNs takes FP64 sums in pass 5.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -51,7 +64,9 @@ namespace heomgb {
 namespace {
 
 constexpr int kDigits = 7, kBits = 9;
-constexpr int kSplitThreads = 320;
+constexpr int kSplitX = 128, kSplitY = 320;  // threads of the two groups
+constexpr int kSplitThreads = kSplitX + kSplitY;
+constexpr int kBarX = 1, kBarY = 2, kBarFull = 3, kBarFree = 4;  // named barriers
 constexpr int kSplitCols = 256;  // tensor-memory columns of a CTA: seven orders of at most 32
 // the digits' bias: sum of 256 * 2^(9 k)
 constexpr unsigned long long kBias = 0x4020100804020100ull;
@@ -69,12 +84,13 @@ __host__ __device__ __forceinline__ SplitGeom split_geom(int n) {
   g.dstride = (g.rows + 7) / 8 * g.sbo;
   return g;
 }
-// the A operand (the last digit's MMA reads 128 rows), later the products
+// the A operand (the last digit's MMA reads 128 rows), then the products
 __host__ __device__ __forceinline__ size_t split_a_bytes(int n) {
   const SplitGeom g = split_geom(n);
-  const size_t a = static_cast<size_t>(kDigits - 1) * g.dstride + 16 * static_cast<size_t>(g.sbo);
-  const size_t p = static_cast<size_t>(g.rows) * (n + 1) * 16;
-  return ((a > p ? a : p) + 127) & ~size_t(127);
+  return (static_cast<size_t>(kDigits - 1) * g.dstride + 16 * static_cast<size_t>(g.sbo) + 127) & ~size_t(127);
+}
+__host__ __device__ __forceinline__ size_t split_p_bytes(int n) {
+  return (static_cast<size_t>(split_geom(n).rows) * (n + 1) * 8 + 127) & ~size_t(127);
 }
 __host__ __device__ __forceinline__ size_t split_b_bytes(int n) {
   const SplitGeom g = split_geom(n);
@@ -106,11 +122,59 @@ __device__ __forceinline__ uint32_t digit_pair(uint32_t a, uint32_t b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// the eight columns of one order at taddr, without the wait
-__device__ __forceinline__ void ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+}
+
+// x != 0 on the bit patterns (a comparison takes the FP64 pipe)
+__device__ __forceinline__ bool nonzero_bits(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+// v 2^e as the nearest double (ties to even), |v| < 2^62 and the result normal:
+// about 20 integer instructions, where a conversion and a multiplication take
+// the FP64 pipe for 128 cycles a warp
+__device__ __forceinline__ double from_fixed(long long v, int e) {
+  const unsigned long long s = static_cast<unsigned long long>(v) & (1ull << 63);
+  unsigned long long m = static_cast<unsigned long long>(v < 0 ? -v : v);
+  if (m == 0ull) return 0.0;
+  const int lz = __clzll(static_cast<long long>(m)) - 1;  // the leading bit to position 62
+  m <<= lz;
+  m = (m + 0x1ffull + ((m >> 10) & 1ull)) >> 10;  // 53 bits; a carry into bit 53 raises the exponent below
+  const unsigned long long ex = static_cast<unsigned long long>(1023 + 62 - lz + e - 1);
+  return __longlong_as_double(static_cast<long long>(s | ((ex << 52) + m)));
+}
+
+// four columns of one order at taddr, without the wait
+__device__ __forceinline__ void ld4_issue(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(taddr));
+}
+
+template <int ID, int COUNT>
+__device__ __forceinline__ void bar_sync() {
+  asm volatile("bar.sync %0, %1;\n" ::"n"(ID), "n"(COUNT) : "memory");
+}
+template <int ID, int COUNT>
+__device__ __forceinline__ void bar_arrive() {
+  asm volatile("bar.arrive %0, %1;\n" ::"n"(ID), "n"(COUNT) : "memory");
+}
+
+__device__ __forceinline__ void split_cp(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s_addr(dst)), "l"(src) : "memory");
+}
+// Issues the copies of a tile's stage input and records (first group).
+__device__ __forceinline__ void split_stage(const DiagInst* __restrict__ I, const DiagTile& td,
+                                            const double2* __restrict__ y, unsigned char* raw) {
+  const int n2 = I->n2, w1 = 1 + I->site_w;
+  double2* ys = reinterpret_cast<double2*>(raw);
+  int4* rec = reinterpret_cast<int4*>(ys + static_cast<size_t>(I->tile) * n2);
+  const double2* ysrc = y + I->elem_off + static_cast<size_t>(td.l0) * n2;
+  const int4* rsrc = I->site_rec + static_cast<size_t>(td.l0) * w1;
+  for (int i = threadIdx.x; i < td.nt * n2; i += kSplitX) split_cp(ys + i, ysrc + i);
+  for (int i = threadIdx.x; i < td.nt * w1; i += kSplitX) split_cp(rec + i, rsrc + i);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
 template <int KIND>
@@ -118,7 +182,8 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tslot;
-  __shared__ unsigned int s_max[8];
+  __shared__ unsigned int s_max3[3][8];  // the largest exponents of a tile's ADOs, three tiles in turn
+  __shared__ volatile int s_fail;  // 1 + the tile whose MMAs did not complete
   double dt;
   int cur;
   // one verdict per CTA (k_rhs_diag_tc)
@@ -126,221 +191,299 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
   const double2* __restrict__ y = stage_input<double2>(st, cur);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned char* As = smem_raw;
-  longlong2* P = reinterpret_cast<longlong2*>(smem_raw);
+  long long* P = reinterpret_cast<long long*>(smem_raw + ds.split_p);
   unsigned char* Bs = smem_raw + ds.split_b;
   if (warp == 0) tmem_alloc(&tslot, kSplitCols);
   if (tid == 0) {
     mbar_init(&mbar);
     mbar_init_fence();
   }
-  if (tid < 8) s_max[tid] = 0u;
+  if (tid < 24) s_max3[tid >> 3][tid & 7] = 0u;
+  if (tid == 0) s_fail = 0;
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = tslot;
-  uint32_t parity = 0;
-  int b_inst = -1;
-  bool fail = false;
   double local = 0.0;
-  for (int t = blockIdx.x; t < ds.n_tiles; t += gridDim.x) {
-    const DiagTile td = ds.tiles[t];
-    const DiagInst* __restrict__ I = ds.inst + td.inst;
-    const int n = I->n, n2 = n * n, K = I->K, w1 = 1 + I->site_w, void_idx = I->nh;
-    const SplitGeom g = split_geom(n);
-    const int l0 = td.l0, nt = td.nt, ne = nt * n2;
-    const double2* __restrict__ yi = y + I->elem_off;
-    double2* ys = reinterpret_cast<double2*>(smem_raw + ds.split_y);
-    int4* rec = reinterpret_cast<int4*>(ys + static_cast<size_t>(g.tile) * n2);
-    // pass 1
-    const double2* ysrc = yi + static_cast<size_t>(l0) * n2;
-    for (int i = tid; i < ne; i += kSplitThreads) ys[i] = __ldg(ysrc + i);
-    for (int i = tid; i < nt * w1; i += kSplitThreads) rec[i] = __ldg(I->site_rec + static_cast<size_t>(l0) * w1 + i);
-    if (td.inst != b_inst) {
-      const int nb = static_cast<int>(split_b_bytes(n) / 16);
-      for (int i = tid; i < nb; i += kSplitThreads) reinterpret_cast<uint4*>(Bs)[i] = __ldg(I->h_digits + i);
-      b_inst = td.inst;
+  const int step = gridDim.x;
+  if (tid < kSplitX) {
+    // ---------------------------------------------------------------- first group: passes 1 to 4
+    uint32_t parity = 0;
+    int b_inst = -1, buf = 0;
+    DiagTile td{}, tdn{};
+    if (blockIdx.x < ds.n_tiles) {
+      tdn = ds.tiles[blockIdx.x];
+      split_stage(ds.inst + tdn.inst, tdn, y, smem_raw + ds.split_y);
     }
-    const int n8 = (n + 7) & ~7, cores = (g.kp - n8) >> 3;  // whole core matrices of K padding
-    for (int q = tid; q < kDigits * nt * 4 * n * cores; q += kSplitThreads) {
-      const int m = q % (nt * 4 * n), r = q / (nt * 4 * n), c = r % cores, d = r / cores;
-      *reinterpret_cast<uint4*>(As + d * g.dstride + (m >> 3) * g.sbo + ((n8 >> 3) + c) * 128 + (m & 7) * 16) =
-          make_uint4(0u, 0u, 0u, 0u);
-    }
-    __syncthreads();
-    for (int lt = 0; lt < nt; ++lt) {
-      unsigned int top = 0u;
-      for (int e = tid; e < n2; e += kSplitThreads) {
-        const double2 v = ys[lt * n2 + e];
-        top = max(top, max(static_cast<unsigned int>(__double2hiint(v.x)) & 0x7fffffffu,
-                                 static_cast<unsigned int>(__double2hiint(v.y)) & 0x7fffffffu));
-      }
-      top = __reduce_max_sync(0xffffffffu, top);
-      if (lane == 0) atomicMax(&s_max[lt], top);
-    }
-    __syncthreads();
-    // pass 2: 2 x 2 blocks of one component, 16 of them an 8 x 8 block
-    {
-      const int nb8 = n8 >> 3, per = 2 * nb8 * nb8 * 16;
-      for (int q = tid; q < nt * per; q += kSplitThreads) {
-        const int lt = q / per, r = q - lt * per, s16 = r & 15, sb = r >> 4;
-        const int comp = sb & 1, b8 = sb >> 1, A8 = b8 / nb8, C8 = b8 - A8 * nb8;
-        const int a = A8 * 8 + (s16 >> 2) * 2, c = C8 * 8 + (s16 & 3) * 2;
-        if (a >= n && c >= n) continue;
-        const int es = max(static_cast<int>(s_max[lt] >> 20), 223);
-        const double* src = reinterpret_cast<const double*>(ys + lt * n2) + comp;
-        unsigned long long v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int aj = a + (j >> 1), cj = c + (j & 1);
-          const double x = aj < n && cj < n ? src[2 * (aj * n + cj)] : 0.0;
-          v[j] = static_cast<unsigned long long>(to_fixed(x, es)) + kBias;
+    for (int t = blockIdx.x; t < ds.n_tiles; t += step, buf = buf == 2 ? 0 : buf + 1) {
+      td = tdn;
+      const DiagInst* __restrict__ I = ds.inst + td.inst;
+      const int n = I->n, n2 = n * n;
+      const SplitGeom g = split_geom(n);
+      const int nt = td.nt, ne = nt * n2;
+      const double2* ys = reinterpret_cast<const double2*>(smem_raw + ds.split_y + buf * ds.split_ybuf);
+      const float r_n2 = 1.0f / n2;
+      unsigned int* s_max = s_max3[buf];
+      // pass 1: the tile (in flight since the last one) has landed; a thread looks at what it copied
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      {
+        unsigned int top = 0u;
+        int lt = 0;
+        for (int i = tid; i < ne; i += kSplitX) {
+          const double2 v = ys[i];
+          const unsigned int m = max(static_cast<unsigned int>(__double2hiint(v.x)) & 0x7fffffffu,
+                                     static_cast<unsigned int>(__double2hiint(v.y)) & 0x7fffffffu);
+          const int li = nt > 1 ? small_div(i, r_n2) : 0;
+          if (li != lt) {
+            atomicMax(&s_max[lt], top);
+            top = 0u;
+            lt = li;
+          }
+          top = max(top, m);
         }
-        const int m = lt * 4 * n + comp * n, mt = m + 2 * n;
-        auto at = [&](int row, int k) { return As + (row >> 3) * g.sbo + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2; };
-        unsigned char *r0 = at(m + a, c), *r1 = at(m + a + 1, c), *t0 = at(mt + c, a), *t1 = at(mt + c + 1, a);
-#pragma unroll
-        for (int d = 0; d < kDigits; ++d) {
-          const int k = kDigits - 1 - d;
-          const uint32_t h0 = digit_pair(digit(v[0], k), digit(v[1], k)), h1 = digit_pair(digit(v[2], k), digit(v[3], k));
-          const int o = d * g.dstride;
-          if (a < n) *reinterpret_cast<uint32_t*>(r0 + o) = h0;
-          if (a + 1 < n) *reinterpret_cast<uint32_t*>(r1 + o) = h1;
-          if (c < n) *reinterpret_cast<uint32_t*>(t0 + o) = __byte_perm(h0, h1, 0x5410);
-          if (c + 1 < n) *reinterpret_cast<uint32_t*>(t1 + o) = __byte_perm(h0, h1, 0x7632);
+        if (nt == 1) {
+          top = __reduce_max_sync(0xffffffffu, top);
+          if (lane == 0) atomicMax(&s_max[0], top);
+        } else {
+          atomicMax(&s_max[lt], top);
         }
       }
-    }
-    fence_async();
-    fence_before();
-    __syncthreads();
-    fence_after();
-    // pass 3
-    if (warp == 0) {
-      if (elect_one()) {
-        const uint32_t a0 = s_addr(As), b0 = s_addr(Bs);
-        for (int d = 0; d < kDigits; ++d) {
-          const int nn = (kDigits - d) * g.np;
-          // D FP32, A and B FP16, both K-major, M = 128
-          const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(nn >> 3) << 17) | (8u << 24);
-          for (int s = 0; s < g.kp / 16; ++s)
-            g_mma(tmem + d * g.np, g_desc(a0 + d * g.dstride + s * 256, 128, g.sbo), g_desc(b0 + s * 256, 128, g.sbo),
-                  idesc, d > 0 || s > 0 ? 1 : 0);
+      const int n8 = (n + 7) & ~7;
+      if (td.inst != b_inst) {  // H's digits, and the K padding of A
+        const int nb = static_cast<int>(split_b_bytes(n) / 16);
+        for (int i = tid; i < nb; i += kSplitX) reinterpret_cast<uint4*>(Bs)[i] = __ldg(I->h_digits + i);
+        if (g.kp > n8) {  // one core matrix: K is n padded to 16
+          const int m = tid & 127;
+          if (m < g.rows)
+            for (int d = tid >> 7; d < kDigits; d += kSplitX / 128)
+              *reinterpret_cast<uint4*>(As + d * g.dstride + (m >> 3) * g.sbo + (n8 >> 3) * 128 + (m & 7) * 16) =
+                  make_uint4(0u, 0u, 0u, 0u);
         }
-        g_commit(&mbar);
+        b_inst = td.inst;
       }
-      __syncwarp();
-    }
-    const uint32_t done = g_wait(&mbar, parity);
-    parity ^= 1u;
-    if (!__syncthreads_and(done)) {
-      if (tid == 0 && st.ctl) st.ctl->status = 2;  // tensor-core wait gave up
-      fail = true;
-      break;
-    }
-    fence_after();
-    // pass 4: warps w and w + 4 read the lanes of sub-partition w, every other block of eight columns
-    if (warp < 8 && (warp & 3) * 32 < nt * 4 * n) {
-      const int m = (warp & 3) * 32 + lane;
-      for (int cb = warp >> 2; cb < n8 >> 3; cb += 2) {
-        uint32_t f[kDigits][8];
+      bar_sync<kBarX, kSplitX>();
+      // pass 2: 2 x 2 blocks of one component, 16 of them an 8 x 8 block
+      {
+        const int nb8 = n8 >> 3, per = 2 * nb8 * nb8 * 16;
+        const float r_per = 1.0f / per, r_nb = 1.0f / nb8;
+        for (int q = tid; q < nt * per; q += kSplitX) {
+          const int lt = small_div(q, r_per), r = q - lt * per, s16 = r & 15, sb = r >> 4;
+          const int comp = sb & 1, b8 = sb >> 1, A8 = small_div(b8, r_nb), C8 = b8 - A8 * nb8;
+          const int a = A8 * 8 + (s16 >> 2) * 2, c = C8 * 8 + (s16 & 3) * 2;
+          if (a >= n && c >= n) continue;
+          const int es = max(static_cast<int>(s_max[lt] >> 20), 223);
+          const double* src = reinterpret_cast<const double*>(ys + lt * n2) + comp;
+          unsigned long long v[4];
 #pragma unroll
-        for (int d = 0; d < kDigits; ++d)
-          ld8_issue(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(d * g.np + cb * 8), f[d]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+          for (int j = 0; j < 4; ++j) {
+            const int aj = a + (j >> 1), cj = c + (j & 1);
+            const double x = aj < n && cj < n ? src[2 * (aj * n + cj)] : 0.0;
+            v[j] = static_cast<unsigned long long>(to_fixed(x, es)) + kBias;
+          }
+          const int m = lt * 4 * n + comp * n, mt = m + 2 * n;
+          auto at = [&](int row, int k) { return As + (row >> 3) * g.sbo + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2; };
+          unsigned char *r0 = at(m + a, c), *r1 = at(m + a + 1, c), *t0 = at(mt + c, a), *t1 = at(mt + c + 1, a);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          long long o[kDigits];
-#pragma unroll
-          for (int d = 0; d < kDigits; ++d) o[d] = __float2int_rn(__uint_as_float(f[d][j]));
-          const long long hi = (o[0] << 18) + (o[1] << 9) + o[2];
-          const long long lo = (o[3] << 27) + (o[4] << 18) + (o[5] << 9) + o[6];
-          if (m < nt * 4 * n && cb * 8 + j < n) P[m * (n + 1) + cb * 8 + j] = make_longlong2(hi, lo);
-        }
-      }
-    }
-    fence_before();
-    __syncthreads();
-    // pass 5
-    const bool sqn = I->sqrt_norm != 0;
-    const size_t g0 = static_cast<size_t>(I->elem_off) + static_cast<size_t>(l0) * n2;
-    const float r_n2 = 1.0f / n2, r_n = 1.0f / n;
-    for (int i = tid; i < ne; i += kSplitThreads) {
-      const int lt = small_div(i, r_n2), e = i - lt * n2, a = small_div(e, r_n), b = e - a * n, l = l0 + lt;
-      const EpiPre pre = epi_pre<double, KIND>(st, g0 + i, cur);
-      const int ex = static_cast<int>(s_max[lt] >> 20), es = max(ex, 223);
-      double2 acc;
-      if (ex <= 1922) {
-        const longlong2* Pl = P + lt * 4 * n * (n + 1);
-        const longlong2 rx = Pl[a * (n + 1) + b], ry = Pl[(n + a) * (n + 1) + b];
-        const longlong2 tx = Pl[(2 * n + b) * (n + 1) + a], ty = Pl[(3 * n + b) * (n + 1) + a];
-        // units of lo: 2^u; a 64-bit integer v with |v| < 2^51 times 2^u is (1.5 2^(52+u) + v 2^u) - 1.5 2^(52+u)
-        const int u = es - 1022 + I->h_exp - 68;
-        const long long ml = (static_cast<long long>(1075 + u) << 52) | (1ll << 51);
-        const long long mh = ml + (36ll << 52);
-        const double cl = __longlong_as_double(ml), ch = __longlong_as_double(mh);
-        acc.x = (__longlong_as_double(mh + (tx.x - rx.x)) - ch) + (__longlong_as_double(ml + (tx.y - rx.y)) - cl);
-        acc.y = (__longlong_as_double(mh + (ty.x - ry.x)) - ch) + (__longlong_as_double(ml + (ty.y - ry.y)) - cl);
-      } else {  // out of the fixed-point range
-        acc = make_double2(0.0, 0.0);
-        const double2* yl = ys + lt * n2;
-        for (int c = 0; c < n; ++c) {
-          const double hac = I->H[a * n + c].x, hcb = I->H[c * n + b].x;
-          const double2 ycb = yl[c * n + b], yac = yl[a * n + c];
-          acc.x = fma(hac, ycb.x, acc.x);
-          acc.x = fma(-hcb, yac.x, acc.x);
-          acc.y = fma(hac, ycb.y, acc.y);
-          acc.y = fma(-hcb, yac.y, acc.y);
+          for (int d = 0; d < kDigits; ++d) {
+            const int k = kDigits - 1 - d;
+            const uint32_t h0 = digit_pair(digit(v[0], k), digit(v[1], k)), h1 = digit_pair(digit(v[2], k), digit(v[3], k));
+            const int o = d * g.dstride;
+            if (a < n) *reinterpret_cast<uint32_t*>(r0 + o) = h0;
+            if (a + 1 < n) *reinterpret_cast<uint32_t*>(r1 + o) = h1;
+            if (c < n) *reinterpret_cast<uint32_t*>(t0 + o) = __byte_perm(h0, h1, 0x5410);
+            if (c + 1 < n) *reinterpret_cast<uint32_t*>(t1 + o) = __byte_perm(h0, h1, 0x7632);
+          }
         }
       }
-      double2 D = make_double2(-acc.y, acc.x);
-      const double2 d0 = __ldg(I->ngd + l), d1 = __ldg(I->c_sd + e);
-      cfma(D, make_double2(d0.x + d1.x, d0.y + d1.y), ys[i]);
-      const int4* rl = rec + lt * w1;
-      const int4 hdr = *rl;
-      if (hdr.y && a != b) {  // +1 terms, the two sites' modes in increasing k
-        const int* p1r = I->p1 + static_cast<size_t>(l) * K;
-        int pa = __ldg(I->site_ptr + a), pb = __ldg(I->site_ptr + b);
-        const int pa1 = __ldg(I->site_ptr + a + 1), pb1 = __ldg(I->site_ptr + b + 1);
-        while (pa < pa1 || pb < pb1) {
-          const int ka = pa < pa1 ? __ldg(I->site_modes + pa) : 0x7fffffff;
-          const int kb = pb < pb1 ? __ldg(I->site_modes + pb) : 0x7fffffff;
-          const bool row = ka < kb;
-          const int k = row ? ka : kb;
-          pa += row ? 1 : 0;
-          pb += row ? 0 : 1;
-          const int lp = __ldg(p1r + k);
-          double2 c = __ldg(I->site_cp2_d + 2 * k + (row ? 0 : 1));
-          if (lp != void_idx && (c.x != 0.0 || c.y != 0.0)) {
-            if (sqn) {
-              const double f = sqrt(static_cast<double>(__ldg(I->nidx + static_cast<size_t>(l) * K + k) + 1));
-              c = make_double2(f * c.x, f * c.y);
+      fence_async();
+      fence_before();
+      bar_sync<kBarX, kSplitX>();
+      fence_after();
+      // pass 3
+      if (warp == 0) {
+        if (elect_one()) {
+          const uint32_t a0 = s_addr(As), b0 = s_addr(Bs);
+          for (int d = 0; d < kDigits; ++d) {
+            const int nn = (kDigits - d) * g.np;
+            // D FP32, A and B FP16, both K-major, M = 128
+            const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(nn >> 3) << 17) | (8u << 24);
+            for (int s = 0; s < g.kp / 16; ++s)
+              g_mma(tmem + d * g.np, g_desc(a0 + d * g.dstride + s * 256, 128, g.sbo), g_desc(b0 + s * 256, 128, g.sbo),
+                    idesc, d > 0 || s > 0 ? 1 : 0);
+          }
+          g_commit(&mbar);
+        }
+        __syncwarp();
+      }
+      if (!g_wait(&mbar, parity)) s_fail = t + 1;  // the tensor-core wait gave up
+      parity ^= 1u;
+      if (t != blockIdx.x) bar_sync<kBarFree, kSplitThreads>();  // the second group has read the last products
+      // the second group is past the tile before the last one, whose buffer takes the next input
+      const int nb = buf == 2 ? 0 : buf + 1;
+      if (t + step < ds.n_tiles && tid < 8) s_max3[nb][tid] = 0u;
+      bar_sync<kBarX, kSplitX>();
+      if (s_fail == t + 1) {
+        bar_arrive<kBarFull, kSplitThreads>();  // the second group leaves too
+        g_wait(&mbar, parity ^ 1u);             // what is in flight drains (bounded) before the tensor memory goes
+        break;
+      }
+      fence_after();
+      if (t + step < ds.n_tiles) {
+        tdn = ds.tiles[t + step];
+        split_stage(ds.inst + tdn.inst, tdn, y, smem_raw + ds.split_y + nb * ds.split_ybuf);
+      }
+      // pass 4: warp w reads the lanes of sub-partition w % 4, in blocks of four columns
+      if ((warp & 3) * 32 < nt * 4 * n) {
+        const int m = (warp & 3) * 32 + lane;
+        for (int cb = warp >> 2; 4 * cb < n; cb += kSplitX / 128) {
+          uint32_t f[kDigits][4];
+#pragma unroll
+          for (int d = 0; d < kDigits; ++d)
+            ld4_issue(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(d * g.np + cb * 4), f[d]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            int o[kDigits];
+#pragma unroll
+            for (int d = 0; d < kDigits; ++d) o[d] = __float2int_rn(__uint_as_float(f[d][j]));
+            const long long hi = mad_wide(o[0], 1 << 18, mad_wide(o[1], 1 << 9, o[2]));
+            const long long lo = mad_wide(o[3], 1 << 27, mad_wide(o[4], 1 << 18, mad_wide(o[5], 1 << 9, o[6])));
+            if (m < nt * 4 * n && cb * 4 + j < n) P[m * (n + 1) + cb * 4 + j] = (hi << 22) + (lo >> 14);
+          }
+        }
+      }
+      fence_before();
+      bar_arrive<kBarFull, kSplitThreads>();
+    }
+  } else {
+    // ---------------------------------------------------------------- second group: passes 5 to 7
+    const int ty = tid - kSplitX;
+    int buf = 0;
+    for (int t = blockIdx.x; t < ds.n_tiles; t += step, buf = buf == 2 ? 0 : buf + 1) {
+      const DiagTile td = ds.tiles[t];
+      const DiagInst* __restrict__ I = ds.inst + td.inst;
+      const int n = I->n, n2 = n * n, K = I->K, w = I->site_w, w1 = 1 + w, void_idx = I->nh, tile = I->tile;
+      const int l0 = td.l0, nt = td.nt, ne = nt * n2;
+      const double2* __restrict__ yi = y + I->elem_off;
+      double2* ys = reinterpret_cast<double2*>(smem_raw + ds.split_y + buf * ds.split_ybuf);
+      const int4* rec = reinterpret_cast<const int4*>(ys + static_cast<size_t>(tile) * n2);
+      const float r_n2 = 1.0f / n2, r_n = 1.0f / n;
+      const unsigned int* s_max = s_max3[buf];
+      bar_sync<kBarFull, kSplitThreads>();
+      if (s_fail == t + 1) break;  // a later tile's failure does not concern this one
+      // pass 5
+      const bool sqn = I->sqrt_norm != 0;
+      const size_t g0 = static_cast<size_t>(I->elem_off) + static_cast<size_t>(l0) * n2;
+      // the neighbour value of the thread's first -1 term is in flight during pass 5
+      // task q of pass 6: mode m of ADO lt (the q-th of w * 2 n places), element e; -1: none
+      const float r_task = 1.0f / (w * 2 * n);
+      auto task = [&](int q, int& lt, int& m) {
+        lt = small_div(q, r_task);
+        const int r = q - lt * (w * 2 * n);
+        m = small_div(r, 0.5f * r_n);
+        const int4* rl = rec + lt * w1;
+        if (lt >= nt || m >= rl->x) return -1;
+        const int j = r - m * 2 * n, s = rl[1 + m].w, a = j < n ? s : j - n, b = j < n ? j : s;
+        if (j >= n && a == s) return -1;
+        for (int p = 0; p < m; ++p)
+          if (rl[1 + p].w == a || rl[1 + p].w == b) return -1;
+        return a * n + b;
+      };
+      auto minus_coef = [&](const int4& r, int a, int b) {
+        return __ldg(I->site_cmn_d + (3 * r.x + (r.w == a ? (r.w == b ? 2 : 0) : 1)) * I->occ_rows + r.z);
+      };
+      int lt_q = 0, m_q = 0;
+      const int e_q = task(ty, lt_q, m_q);
+      double2 v_q = make_double2(0.0, 0.0);
+      if (e_q >= 0) v_q = __ldg(yi + static_cast<size_t>(rec[lt_q * w1 + 1 + m_q].y) * n2 + e_q);
+      for (int i = ty; i < ne; i += kSplitY) {
+        const int lt = small_div(i, r_n2), e = i - lt * n2, a = small_div(e, r_n), b = e - a * n, l = l0 + lt;
+        const int ex = static_cast<int>(s_max[lt] >> 20), es = max(ex, 223);
+        double2 acc;
+        if (ex <= 1922) {
+          const long long* Pl = P + lt * 4 * n * (n + 1);
+          const long long vx = Pl[(2 * n + b) * (n + 1) + a] - Pl[a * (n + 1) + b];
+          const long long vy = Pl[(3 * n + b) * (n + 1) + a] - Pl[(n + a) * (n + 1) + b];
+          const int u = es - 1022 + I->h_exp - 54;
+          acc.x = from_fixed(vx, u);
+          acc.y = from_fixed(vy, u);
+        } else {  // out of the fixed-point range
+          acc = make_double2(0.0, 0.0);
+          const double2* __restrict__ yl = yi + static_cast<size_t>(l) * n2;  // ys is being replaced
+          for (int c = 0; c < n; ++c) {
+            const double hac = I->H[a * n + c].x, hcb = I->H[c * n + b].x;
+            const double2 ycb = __ldg(yl + c * n + b), yac = __ldg(yl + a * n + c);
+            acc.x = fma(hac, ycb.x, acc.x);
+            acc.x = fma(-hcb, yac.x, acc.x);
+            acc.y = fma(hac, ycb.y, acc.y);
+            acc.y = fma(-hcb, yac.y, acc.y);
+          }
+        }
+        double2 D = make_double2(-acc.y, acc.x);
+        // damping
+        const double2 d0 = __ldg(I->ngd + l), d1 = __ldg(I->c_sd + e), yv = ys[i];
+        cfma(D, make_double2(d0.x + d1.x, d0.y + d1.y), yv);
+        if (rec[lt * w1].y && a != b) {  // +1 terms, the two sites' modes in increasing k
+          const int* p1r = I->p1 + static_cast<size_t>(l) * K;
+          int pa = __ldg(I->site_ptr + a), pb = __ldg(I->site_ptr + b);
+          const int pa1 = __ldg(I->site_ptr + a + 1), pb1 = __ldg(I->site_ptr + b + 1);
+          while (pa < pa1 || pb < pb1) {
+            const int ka = pa < pa1 ? __ldg(I->site_modes + pa) : 0x7fffffff;
+            const int kb = pb < pb1 ? __ldg(I->site_modes + pb) : 0x7fffffff;
+            const bool row = ka < kb;
+            const int k = row ? ka : kb;
+            pa += row ? 1 : 0;
+            pb += row ? 0 : 1;
+            const int lp = __ldg(p1r + k);
+            double2 c = __ldg(I->site_cp2_d + 2 * k + (row ? 0 : 1));
+            if (lp != void_idx && (nonzero_bits(c.x) || nonzero_bits(c.y))) {
+              if (sqn) {
+                const double f = sqrt(static_cast<double>(__ldg(I->nidx + static_cast<size_t>(l) * K + k) + 1));
+                c = make_double2(f * c.x, f * c.y);
+              }
+              cfma(D, c, __ldg(yi + static_cast<size_t>(lp) * n2 + e));
             }
-            cfma(D, c, __ldg(yi + static_cast<size_t>(lp) * n2 + e));
           }
         }
+        ys[i] = D;  // the element's input is spent
       }
-      for (int q = 1; q <= hdr.x; ++q) {  // -1 terms: the ADO's occupied modes
-        const int4 r = rl[q];              // k, ptr_m1, n_k, site
-        if (r.w == a || r.w == b) {
-          const double2 c = __ldg(I->site_cm3_d + 3 * r.x + (r.w == a ? (r.w == b ? 2 : 0) : 1));
-          if (c.x != 0.0 || c.y != 0.0) {
-            const double f = sqn ? sqrt(static_cast<double>(r.z)) : occ<double>(r.z);
-            cfma(D, make_double2(f * c.x, f * c.y), __ldg(yi + static_cast<size_t>(r.y) * n2 + e));
+      bar_sync<kBarY, kSplitY>();
+      if (t + step < ds.n_tiles) bar_arrive<kBarFree, kSplitThreads>();  // the products are read
+      // pass 6: the -1 terms of the occupied modes.  A mode touches 2 n - 1 elements of its ADO;
+      // the thread of an element's first mode adds the terms of all
+      for (int q = ty; q < nt * w * 2 * n; q += kSplitY) {
+        int lt = lt_q, m = m_q, e = e_q;
+        double2 v = v_q;
+        if (q != ty) {
+          e = task(q, lt, m);
+          if (e >= 0) v = __ldg(yi + static_cast<size_t>(rec[lt * w1 + 1 + m].y) * n2 + e);
+        }
+        if (e < 0) continue;
+        const int4* rl = rec + lt * w1;
+        const int a = small_div(e, r_n), b = e - a * n, nm = rl->x;
+        double2 D = ys[lt * n2 + e];
+        for (int p = m; p < nm; ++p) {
+          const int4 r = rl[1 + p];  // k, ptr_m1, n_k, site
+          if (r.w == a || r.w == b) {
+            const double2 c = minus_coef(r, a, b);
+            if (p > m) v = __ldg(yi + static_cast<size_t>(r.y) * n2 + e);
+            if (nonzero_bits(c.x) || nonzero_bits(c.y)) cfma(D, c, v);
           }
         }
+        ys[lt * n2 + e] = D;
       }
-      local += epi_post<double, KIND>(st, g0 + i, D, dt, cur, pre);
+      bar_sync<kBarY, kSplitY>();
+      // pass 7: stage epilogue
+      for (int i = ty; i < ne; i += kSplitY) {
+        const EpiPre p = epi_pre<double, KIND>(st, g0 + i, cur);
+        local += epi_post<double, KIND>(st, g0 + i, ys[i], dt, cur, p);
+      }
     }
-    __syncthreads();  // the products, the input and the maxima are free
-    if (tid < 8) s_max[tid] = 0u;
-  }
-  if (fail) {
-    g_wait(&mbar, parity ^ 1u);  // what is in flight drains (bounded) before the tensor memory goes
-    __syncthreads();
   }
   fence_before();
   __syncthreads();
   fence_after();
+  if (s_fail && tid == 0 && st.ctl) st.ctl->status = 2;
   if (warp == 0) tmem_free(tmem, kSplitCols);
   if (KIND == EPI_DP7) dp7_finish(st, local, ds.total);
 }
@@ -401,8 +544,9 @@ bool split_eligible(const DiagInst& I, bool mixed) {
 
 int split_tile(int n) { return split_geom(n).tile; }
 
-void split_smem(const DiagInst& I, size_t* a, size_t* b, size_t* y) {
+void split_smem(const DiagInst& I, size_t* a, size_t* p, size_t* b, size_t* y) {
   *a = split_a_bytes(I.n);
+  *p = split_p_bytes(I.n);
   *b = split_b_bytes(I.n);
   *y = split_y_bytes(I.n, I.site_w);
 }

@@ -14,10 +14,12 @@
 // left out (orders above 6 and bits of rho below 2^-62 of the ADO's largest)
 // is below 2^-57 of the largest product (the error-free splitting of matrix
 // products of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012).
-// Measured on the 24-site aggregate at depth 3: a state's error against
-// extended precision is 7.0e-17 after 4 steps, 7.6e-17 with the FP64 sums; a
-// stage of 12M elements takes 0.59 ms, 2.95 with k_rhs_diag<double>, whose FP64
-// pipe alone needs 2.58 (16 sites, depth 3: 0.088 and 0.287).
+// Measured against extended precision over aggregates of 4 to 24 sites, states
+// after two steps: 1.34e-16 with either where the step leaves the state's own
+// rounding in charge, 4.0e-16 here and 4.7e-16 with the FP64 sums at 24 sites
+// where the operator is (steps 40 times longer).  A stage of the 24-site model
+// at depth 3 (12M elements) takes 0.59 ms, 2.95 with k_rhs_diag<double>, whose
+// FP64 pipe alone needs 2.58 (16 sites: 0.088 and 0.287).
 //
 // Per tile of T = 128 / (4 n) ADOs, the first group of a CTA (128 threads):
 //   1. the stage input (copied with cp.async a tile ahead), each ADO's largest
@@ -28,7 +30,9 @@
 //      H at once (N = 7 - i blocks of n padded to 16), into the tensor-memory
 //      columns of the orders i..6, so 7 MMAs per 16 of K cover all 28 pairs;
 //   4. read-back: rows of R H, I H (rho H) and R^T H, I^T H (H rho,
-//      transposed) as 64-bit integers (60 bits of each product) in shared memory;
+//      transposed) as 64-bit integers in shared memory, in units of 2^-57 of the
+//      product of the largest elements (a sum of n <= 32 of them, and the
+//      difference of two sums, stay below 2^63);
 // and the second group (320 threads), a tile behind it:
 //   5. one element per thread: the difference of the two products, rounded to
 //      FP64 with integer operations; damping and +1 terms (ADOs below the
@@ -131,7 +135,7 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
 // x != 0 on the bit patterns (a comparison takes the FP64 pipe)
 __device__ __forceinline__ bool nonzero_bits(double x) { return (__double_as_longlong(x) << 1) != 0; }
 
-// v 2^e as the nearest double (ties to even), |v| < 2^62 and the result normal:
+// v 2^e as the nearest double (ties to even), |v| < 2^63 and the result normal:
 // about 20 integer instructions, where a conversion and a multiplication take
 // the FP64 pipe for 128 cycles a warp
 __device__ __forceinline__ double from_fixed(long long v, int e) {
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
             for (int d = 0; d < kDigits; ++d) o[d] = __float2int_rn(__uint_as_float(f[d][j]));
             const long long hi = mad_wide(o[0], 1 << 18, mad_wide(o[1], 1 << 9, o[2]));
             const long long lo = mad_wide(o[3], 1 << 27, mad_wide(o[4], 1 << 18, mad_wide(o[5], 1 << 9, o[6])));
-            if (m < nt * 4 * n && cb * 4 + j < n) P[m * (n + 1) + cb * 4 + j] = (hi << 22) + (lo >> 14);
+            if (m < nt * 4 * n && cb * 4 + j < n) P[m * (n + 1) + cb * 4 + j] = (hi << 25) + ((lo + 1024) >> 11);
           }
         }
       }
@@ -404,7 +408,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
           const long long* Pl = P + lt * 4 * n * (n + 1);
           const long long vx = Pl[(2 * n + b) * (n + 1) + a] - Pl[a * (n + 1) + b];
           const long long vy = Pl[(3 * n + b) * (n + 1) + a] - Pl[(n + a) * (n + 1) + b];
-          const int u = es - 1022 + I->h_exp - 54;
+          const int u = es - 1022 + I->h_exp - 57;
           acc.x = from_fixed(vx, u);
           acc.y = from_fixed(vy, u);
         } else {  // out of the fixed-point range

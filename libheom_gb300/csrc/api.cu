@@ -886,11 +886,7 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
       int4* rec = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));
       di.site_rec = rec;
       ck(launch_site_records(di, dms, rec, s), "site records");
-      if (q->precision_eff == HEOMGB_FP64 && di.h_sym && n >= 4 && n <= 32) {
-        std::vector<double> Hr(n2);
-        for (int e = 0; e < n2; ++e) Hr[e] = H[e].real();
-        const std::vector<unsigned short> dig = split_h_digits(Hr.data(), n, &di.h_exp);
-        if (!dig.empty()) di.h_digits = reinterpret_cast<const uint4*>(q->arena.upload(dig, s));
+      if (q->precision_eff == HEOMGB_FP64) {
         std::vector<cd> cmn(cm3.size() * di.occ_rows);
         for (size_t p = 0; p < cm3.size(); ++p)
           for (int o = 0; o < di.occ_rows; ++o) {
@@ -898,6 +894,12 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
             cmn[p * di.occ_rows + o] = cd(f * cm3[p].real(), f * cm3[p].imag());
           }
         di.site_cmn_d = q->arena.upload(to_d2(cmn), s);
+      }
+      if (q->precision_eff == HEOMGB_FP64 && di.h_sym && n >= 4 && n <= 32) {
+        std::vector<double> Hr(n2);
+        for (int e = 0; e < n2; ++e) Hr[e] = H[e].real();
+        const std::vector<unsigned short> dig = split_h_digits(Hr.data(), n, &di.h_exp);
+        if (!dig.empty()) di.h_digits = reinterpret_cast<const uint4*>(q->arena.upload(dig, s));
       }
       if (rows_eligible(di, q->precision_eff == HEOMGB_MIXED)) {
         int4* rr = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));

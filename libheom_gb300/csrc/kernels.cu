@@ -658,6 +658,7 @@ template <int EPT>
 struct ResElems {
   int lt[EPT], e[EPT], a[EPT], b[EPT];
   int gi[EPT];    // the element's index in the state vector
+  int wc[EPT];    // slots of the bath-term table that any of the warp's elements fills
   float2 g[EPT];  // damping coefficient sum_k n_k gamma_k + the element's s_delta term
 };
 
@@ -684,9 +685,10 @@ __device__ __forceinline__ ResAdos res_ados(int nh) {
 
 // Builds the thread's element data and, for its elements, the bath-term table
 // (slot-major: Toff[j * E + le] the neighbour element's offset in the state,
-// -1 for none, Tcf the coefficient; slots 0-3 hold the +1 terms, 4-7 the -1
-// terms, in k_rhs_diag's order; the host admits models with at most 4 + 4
-// terms per element).
+// -1 for none, Tcf the coefficient; the terms that have a neighbour, +1 then -1
+// in k_rhs_diag's order, fill the slots from the first, so that a warp stops
+// after its fullest element; the host admits models with at most 4 + 4 terms
+// per element).
 template <int EPT>
 __device__ __forceinline__ void res_build(const DiagInst& I, const ResAdos& A, int E, int* Toff, float2* Tcf,
                                           ResElems<EPT>& el) {
@@ -705,7 +707,13 @@ __device__ __forceinline__ void res_build(const DiagInst& I, const ResAdos& A, i
     el.gi[r] = l * n2 + e;
     const float2 g0 = I.ngd_f[l], g1 = I.c_sd_f[e];
     el.g[r] = make_float2(g0.x + g1.x, g0.y + g1.y);
+    int cnt = 0;
     if (le < E) {
+      auto put = [&](int off, float2 cf) {
+        Toff[static_cast<size_t>(cnt) * E + le] = off;
+        Tcf[static_cast<size_t>(cnt) * E + le] = cf;
+        ++cnt;
+      };
       const int* __restrict__ p1row = I.p1 + static_cast<size_t>(l) * K;
       const int* __restrict__ m1row = I.m1 + static_cast<size_t>(l) * K;
       const int* __restrict__ nrow = I.nidx + static_cast<size_t>(l) * K;
@@ -727,8 +735,7 @@ __device__ __forceinline__ void res_build(const DiagInst& I, const ResAdos& A, i
             }
           }
         }
-        Toff[static_cast<size_t>(j) * E + le] = off;
-        Tcf[static_cast<size_t>(j) * E + le] = cf;
+        if (off >= 0) put(off, cf);
       }
       for (int j = 0; j < 4; ++j) {
         int off = -1;
@@ -745,10 +752,14 @@ __device__ __forceinline__ void res_build(const DiagInst& I, const ResAdos& A, i
             cf = make_float2(nk * cm.x, nk * cm.y);
           }
         }
-        Toff[static_cast<size_t>(4 + j) * E + le] = off;
-        Tcf[static_cast<size_t>(4 + j) * E + le] = cf;
+        if (off >= 0) put(off, cf);
       }
+      el.wc[r] = cnt;
+      while (cnt < kResidentTerms) put(-1, make_float2(0.f, 0.f));
+    } else {
+      el.wc[r] = 0;
     }
+    el.wc[r] = __reduce_max_sync(0xffffffffu, el.wc[r]);
   }
 }
 
@@ -808,16 +819,20 @@ __device__ __forceinline__ void res_own(const float2* Hs, const float2* Xs, int 
 // Bath terms of the thread's elements added to D: all neighbour gathers are
 // issued first (L1-bypassing loads of the other CTAs' stage input Xg, which
 // must not be restrict-qualified: it is written until the grid wait returns).
-template <int EPT>
+// A slot beyond the warp's fullest element is skipped (it would add 0 * 0);
+// GUARD: its gather too, a branch that pays where the other loads of the stage
+// are many (7 sites, Dormand-Prince at depth 4: 1.26 ms with it, 1.32 without;
+// RK4 2.64 and 2.78; LSRK4 at depth 3 the other way, 1.83 and 1.73).
+template <int EPT, bool GUARD = true>
 __device__ __forceinline__ void res_bath(const float2* Xg, const int* Toff, const float2* Tcf, int E,
-                                         float2 (&D)[EPT]) {
+                                         const ResElems<EPT>& el, float2 (&D)[EPT]) {
   float2 vv[EPT][kResidentTerms];
 #pragma unroll
   for (int r = 0; r < EPT; ++r) {
     const int le = threadIdx.x + r * blockDim.x;
 #pragma unroll
     for (int j = 0; j < kResidentTerms; ++j) {
-      const int off = le < E ? Toff[static_cast<size_t>(j) * E + le] : -1;
+      const int off = (!GUARD || j < el.wc[r]) && le < E ? Toff[static_cast<size_t>(j) * E + le] : -1;
       vv[r][j] = off >= 0 ? __ldcg(Xg + off) : make_float2(0.f, 0.f);
     }
   }
@@ -826,7 +841,8 @@ __device__ __forceinline__ void res_bath(const float2* Xg, const int* Toff, cons
     const int le = threadIdx.x + r * blockDim.x;
     if (le >= E) continue;
 #pragma unroll
-    for (int j = 0; j < kResidentTerms; ++j) cfma(D[r], Tcf[static_cast<size_t>(j) * E + le], vv[r][j]);
+    for (int j = 0; j < kResidentTerms; ++j)
+      if (j < el.wc[r]) cfma(D[r], Tcf[static_cast<size_t>(j) * E + le], vv[r][j]);
   }
 }
 
@@ -906,7 +922,7 @@ __global__ void __launch_bounds__(kResidentMaxBlock, 2) k_dp_resident(const Resi
           ok = grid_wait(R.bar, gen, R.spin_limit);
           if (!ok) break;
         }
-        res_bath<EPT>(Xg, Toff, Tcf, E, D);
+        res_bath<EPT>(Xg, Toff, Tcf, E, el, D);
         if (s == 0 || s == 6)
 #pragma unroll
           for (int r = 0; r < EPT; ++r) (s == 0 ? D1 : D7)[r] = D[r];
@@ -1044,7 +1060,7 @@ __global__ void __launch_bounds__(kResidentMaxBlock, 2) k_rk4_resident(const Res
         ok = grid_wait(R.bar, gen, R.spin_limit);
         if (!ok) break;
       }
-      res_bath<EPT>(Xg, Toff, Tcf, E, D);
+      res_bath<EPT>(Xg, Toff, Tcf, E, el, D);
 #pragma unroll
       for (int r = 0; r < EPT; ++r) {
         const int le = threadIdx.x + r * blockDim.x;
@@ -1108,7 +1124,13 @@ __device__ __forceinline__ void res_build64(const DiagInst& I, const ResAdos& A,
     el.gi[r] = l * n2 + e;
     const double2 g0 = I.ngd[l], g1 = I.c_sd[e];
     g[r] = make_double2(g0.x + g1.x, g0.y + g1.y);
+    int cnt = 0;
     if (le < E) {
+      auto put = [&](int off, double2 cf) {
+        Toff[static_cast<size_t>(cnt) * E + le] = off;
+        Tcf[static_cast<size_t>(cnt) * E + le] = cf;
+        ++cnt;
+      };
       const int* __restrict__ p1row = I.p1 + static_cast<size_t>(l) * K;
       const int* __restrict__ m1row = I.m1 + static_cast<size_t>(l) * K;
       const int* __restrict__ nrow = I.nidx + static_cast<size_t>(l) * K;
@@ -1130,8 +1152,7 @@ __device__ __forceinline__ void res_build64(const DiagInst& I, const ResAdos& A,
             }
           }
         }
-        Toff[static_cast<size_t>(j) * E + le] = off;
-        Tcf[static_cast<size_t>(j) * E + le] = cf;
+        if (off >= 0) put(off, cf);
       }
       for (int j = 0; j < 4; ++j) {
         int off = -1;
@@ -1148,10 +1169,14 @@ __device__ __forceinline__ void res_build64(const DiagInst& I, const ResAdos& A,
             cf = make_double2(nk * cm.x, nk * cm.y);
           }
         }
-        Toff[static_cast<size_t>(4 + j) * E + le] = off;
-        Tcf[static_cast<size_t>(4 + j) * E + le] = cf;
+        if (off >= 0) put(off, cf);
       }
+      el.wc[r] = cnt;
+      while (cnt < kResidentTerms) put(-1, make_double2(0.0, 0.0));
+    } else {
+      el.wc[r] = 0;
     }
+    el.wc[r] = __reduce_max_sync(0xffffffffu, el.wc[r]);
   }
 }
 
@@ -1241,7 +1266,8 @@ __global__ void __launch_bounds__(kResidentMaxBlock, 2) k_rk4_resident64(const R
         const int le = threadIdx.x + r * blockDim.x;
         if (le >= E) continue;
 #pragma unroll
-        for (int j = 0; j < kResidentTerms; ++j) cfma(D[r], Tcf[static_cast<size_t>(j) * E + le], vv[r][j]);
+        for (int j = 0; j < kResidentTerms; ++j)
+          if (j < el.wc[r]) cfma(D[r], Tcf[static_cast<size_t>(j) * E + le], vv[r][j]);  // warp-uniform
         const double2 k = make_double2(-dt * D[r].x, -dt * D[r].y);
         const size_t g = el.gi[r];
         if (s < 3) {  // rho_n = rho + c*k ; acc = rho + k/6 or acc += k/3
@@ -1314,7 +1340,7 @@ __global__ void __launch_bounds__(kResidentMaxBlock, 2) k_ls_resident(const Resi
       } else {
         __syncthreads();
       }
-      res_bath<EPT>(Xg, Toff, Tcf, E, D);
+      res_bath<EPT, false>(Xg, Toff, Tcf, E, el, D);
 #pragma unroll
       for (int r = 0; r < EPT; ++r) {
         const int le = threadIdx.x + r * blockDim.x;

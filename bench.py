@@ -134,6 +134,14 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
+def stage_kernel(tunings):
+    """The stage kernel that a solver's plan (its parts' plans) runs."""
+    for key in ("sites", "rows", "split"):
+        if any(t.get(key, False) for t in tunings):
+            return "k_rhs_" + key
+    return "k_rhs_diag"
+
+
 def measured_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -359,8 +367,7 @@ def secondary_aggregate24(stream, fma_peaks, steps=3):
         tune = qs.tuning()
         entry = {"value": upd / (statistics.median(ms) / 1e3), "unit": "ADO-updates/s",
                  "ms_per_solve": statistics.median(ms), "avg_stage_kernel_us": 1e6 * avg_s,
-                 "kernel": "k_rhs_sites" if tune.get("sites") else "k_rhs_rows" if tune.get("rows") else "k_rhs_diag",
-                 "tuning": tune}
+                 "kernel": stage_kernel([tune]), "tuning": tune}
         if form == "mixed":
             entry["roofline"] = {"bound": "hbm", "achieved": alg / avg_s / 1e9, "peak": peak, "unit": "GB/s",
                                  "frac": alg / avg_s / 1e9 / peak, "peak_source": peak_kind,
@@ -593,15 +600,17 @@ def run_ours(args):
         kernel = {"rkdp": "k_dp_resident", "rk4": "k_rk4_resident", "lsrk4": "k_ls_resident"}[wl["solver"]] + (
             " (one cooperative launch per output interval: fused RHS and stage epilogues"
             + (", error norm and step control" if wl["solver"] == "rkdp" else "") + "; state in shared memory)")
+    elif any(t.get("cluster", False) for t in part_tunings):
+        kernel = ("k_cluster (one launch per output interval; every bin of instances inside one thread-block cluster"
+                  + (")" if all(t.get("cluster", False) for t in part_tunings)
+                     else "); " + stage_kernel([t for t in part_tunings if not t.get("cluster", False)])
+                     + " or k_fixed_local for the other part"))
     elif local:
         kernel = ("k_fixed_local (one launch per output interval; every instance inside one CTA with its stage "
                   "inputs in shared memory, no grid-wide synchronisation)"
                   + ("" if all(t.get("local", False) for t in part_tunings) else "; k_rhs_diag for the other part"))
     else:
-        kernel = ("k_rhs_sites (site-local baths: fused RHS + stage epilogue)"
-                  if any(t.get("sites", False) for t in part_tunings)
-                  else "k_rhs_rows (site-local baths: fused RHS + stage epilogue)"
-                  if any(t.get("rows", False) for t in part_tunings) else "k_rhs_diag (fused RHS + stage epilogue)")
+        kernel = stage_kernel(part_tunings) + " (fused RHS + stage epilogue)"
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": profile_traffic(args.workload, args.form), "peak_source": peak_kind,
             "kernel": kernel,

@@ -1,6 +1,6 @@
 """Build of the CUDA library libheom_gb300/_lib/libheomgb.so (sm_103a only).
 
-The two translation units compile in parallel with nvcc and link into one
+The translation units compile in parallel with nvcc and link into one
 shared library that exports the C ABI of include/heomgb.h.
 """
 from __future__ import annotations

@@ -1859,6 +1859,10 @@ __global__ void __launch_bounds__(256) k_rhs_general(const RhsModel m, const Sta
 // on ADO n+1_k and n_k (s_k Phi_u - a_k Psi_u) on ADO n-1_k.  The blocks are
 // the shared CSR superoperators scaled by per-ADO scalars, so the block
 // pattern comes from the hierarchy tables and R is never materialised.
+// Baths whose Phi and Psi k_rhs_liou holds at a time, `size` bytes an element
+__host__ __device__ inline int liou_baths(int U, int n2, size_t size) {
+  return U <= 1 ? 1 : size * static_cast<size_t>(n2) * (2 + 2 * static_cast<size_t>(U)) <= 64 * 1024 ? U : 1;
+}
 template <typename TC, typename TB>
 __global__ void __launch_bounds__(256) k_rhs_liou(const RhsModel m, const Stage st) {
   using C = cx_t<TC>;
@@ -1871,7 +1875,8 @@ __global__ void __launch_bounds__(256) k_rhs_liou(const RhsModel m, const Stage 
   C* ys = reinterpret_cast<C*>(smem_raw);
   C* Dm = ys + n2;
   C* TPhi = Dm + n2;
-  C* TPsi = TPhi + n2;
+  const int at = liou_baths(m.U, n2, sizeof(C));
+  C* TPsi = TPhi + static_cast<size_t>(at) * n2;
   const C* __restrict__ ngd = pick<TC>(m.ngd, m.ngd_f);
   const C* __restrict__ r0v = pick<TC>(m.r0_val, m.r0_val_f);
   const C* __restrict__ phv = pick<TC>(m.phi_val, m.phi_val_f);
@@ -1883,17 +1888,14 @@ __global__ void __launch_bounds__(256) k_rhs_liou(const RhsModel m, const Stage 
   for (int l = blockIdx.x; l < m.n_hrchy; l += gridDim.x) {
     const TB* yl = y + static_cast<size_t>(l) * n2;
     for (int e = threadIdx.x; e < n2; e += blockDim.x) ys[e] = ldc<TC>(yl + e);
-    __syncthreads();
-    const C gl = ngd[l];
-    for (int r = threadIdx.x; r < n2; r += blockDim.x) {
-      C D = cx<TC>(0, 0);
-      for (int p = __ldg(m.r0_ptr + r); p < __ldg(m.r0_ptr + r + 1); ++p) cfma(D, r0v[p], ys[__ldg(m.r0_idx + p)]);
-      cfma(D, gl, ys[r]);
-      Dm[r] = D;
-    }
-    for (int u = 0; u < m.U; ++u) {
-      const int k0 = __ldg(m.bath_ptr + u), k1 = __ldg(m.bath_ptr + u + 1);
-      for (int e = threadIdx.x; e < n2; e += blockDim.x) {
+    // the baths `at` a time (liou_baths: all of them where shared memory holds their Phi and Psi,
+    // so that their gathers overlap and one barrier separates them from the products: the chain of
+    // an ADO with every neighbour bounds the stage, 17.9 -> 15.7 us for 7 sites at depth 3)
+    for (int u0 = 0; u0 < m.U || u0 == 0; u0 += at) {
+      const int nu = min(at, m.U - u0);
+      for (int i = threadIdx.x; i < nu * n2; i += blockDim.x) {
+        const int u = u0 + i / n2, e = i % n2;
+        const int k0 = __ldg(m.bath_ptr + u), k1 = __ldg(m.bath_ptr + u + 1);
         C ph = cx<TC>(0, 0), ps = cx<TC>(0, 0);
         for (int k = k0; k < k1; ++k) {
           const int lp = __ldg(m.p1 + static_cast<size_t>(l) * K + k);
@@ -1916,23 +1918,31 @@ __global__ void __launch_bounds__(256) k_rhs_liou(const RhsModel m, const Stage 
             cfma(ps, cx<TC>(-nk * av[k].x, -nk * av[k].y), r);
           }
         }
-        TPhi[e] = ph;
-        TPsi[e] = ps;
+        TPhi[i] = ph;
+        TPsi[i] = ps;
       }
       __syncthreads();
-      const int* pp = m.phi_ptr + static_cast<size_t>(u) * (n2 + 1);
-      const int* qp = m.psi_ptr + static_cast<size_t>(u) * (n2 + 1);
       for (int r = threadIdx.x; r < n2; r += blockDim.x) {
-        C D = Dm[r];
-        for (int p = __ldg(pp + r); p < __ldg(pp + r + 1); ++p) cfma(D, phv[p], TPhi[__ldg(m.phi_idx + p)]);
-        for (int p = __ldg(qp + r); p < __ldg(qp + r + 1); ++p) cfma(D, psv[p], TPsi[__ldg(m.psi_idx + p)]);
-        Dm[r] = D;
+        C D = cx<TC>(0, 0);
+        if (u0 == 0) {
+          for (int p = __ldg(m.r0_ptr + r); p < __ldg(m.r0_ptr + r + 1); ++p) cfma(D, r0v[p], ys[__ldg(m.r0_idx + p)]);
+          cfma(D, ngd[l], ys[r]);
+        } else {
+          D = Dm[r];
+        }
+        for (int j = 0; j < nu; ++j) {
+          const int* pp = m.phi_ptr + static_cast<size_t>(u0 + j) * (n2 + 1);
+          const int* qp = m.psi_ptr + static_cast<size_t>(u0 + j) * (n2 + 1);
+          for (int p = __ldg(pp + r); p < __ldg(pp + r + 1); ++p) cfma(D, phv[p], TPhi[j * n2 + __ldg(m.phi_idx + p)]);
+          for (int p = __ldg(qp + r); p < __ldg(qp + r + 1); ++p) cfma(D, psv[p], TPsi[j * n2 + __ldg(m.psi_idx + p)]);
+        }
+        if (u0 + at >= m.U)
+          local += epilogue<TC>(st, static_cast<size_t>(l) * n2 + r, D, dt, cur);
+        else
+          Dm[r] = D;
       }
       __syncthreads();
     }
-    for (int e = threadIdx.x; e < n2; e += blockDim.x)
-      local += epilogue<TC>(st, static_cast<size_t>(l) * n2 + e, Dm[e], dt, cur);
-    __syncthreads();
   }
   if (st.kind == EPI_DP7) dp7_finish(st, local, static_cast<long long>(m.n_hrchy) * n2);
 }
@@ -2008,8 +2018,10 @@ __global__ void __launch_bounds__(256) k_rhs_redfield(const RhsModel m, const St
 // ------------------------------------------------------------------ launch configuration
 int rhs_block_size(const RhsModel& m, int path) {
   if (path != PATH_DIAG) {
+    // k_rhs_liou forms all its baths' Phi and Psi together
+    const int work = path == PATH_LIOU ? m.n2 * std::max(1, m.U) : m.n2;
     int b = 32;
-    while (b < m.n2 && b < 256) b <<= 1;
+    while (b < work && b < 256) b <<= 1;
     return b;
   }
   return 128;
@@ -2025,7 +2037,7 @@ int rhs_grid_size(const RhsModel& m, int path, int block, int n_sm) {
 size_t rhs_smem_bytes(const RhsModel& m, int path, bool mixed) {
   const size_t cb = mixed ? sizeof(float2) : sizeof(double2);
   if (path == PATH_GENERAL) return 5 * cb * m.n2;
-  if (path == PATH_LIOU) return 4 * cb * m.n2;
+  if (path == PATH_LIOU) return (2 + 2 * static_cast<size_t>(liou_baths(m.U, m.n2, cb))) * cb * m.n2;
   if (path == PATH_REDFIELD) return 3 * cb * m.n2;
   return 0;
 }

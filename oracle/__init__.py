@@ -74,9 +74,14 @@ class PackedCase:
             self.struct.hrchy_filter = ctypes.cast(self.filter, ctypes.c_void_p)
 
 
+def has_ref_tree() -> bool:
+    """Whether the reference's sources are there (its directory may be there and empty)."""
+    return os.path.isdir(os.path.join(REF_TREE, "src"))
+
+
 def build(which: str = "port") -> None:
     target = {"port": PORT_SO, "ref": REF_SO, "ref_sqrt": REF_SQRT_SO}[which]
-    if which.startswith("ref") and not os.path.isdir(REF_TREE):
+    if which.startswith("ref") and not has_ref_tree():
         raise FileNotFoundError("reference tree not present; the reference oracle cannot be built here")
     subprocess.run(["make", "-s", "-C", HERE, "port" if which == "port" else "ref"], check=True)
     if not os.path.exists(target):

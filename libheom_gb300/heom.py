@@ -452,24 +452,37 @@ class batch_solver:
         t = [float(x) for x in t_list]
         self._counts = [dict(rhs=0, attempts=0, accepted=0) for _ in self._parts]
         with ThreadPoolExecutor(len(self._parts)) as pool:  # sub-batches run concurrently (own streams)
-            # nobody looks at rho between the intervals without a callback: one solve covers them all
-            for i in range(len(t) - 1) if callback else range(min(1, len(t) - 1)):
+            if not callback and len(t) > 2 and not isinstance(self.solver, rkdp):
+                # nobody looks at rho between the intervals: one solve covers them all.  Where a
+                # sub-batch fails, rho is as it was, and the solve goes interval by interval
+                # up to the failure, which leaves every instance at the last common time
+                # (Dormand-Prince keeps its step size from one solve to the next, so it
+                # goes interval by interval from the start).
+                try:
+                    self._run(pool, flat, t, kwargs)
+                    return
+                except Exception:
+                    self._counts = [dict(rhs=0, attempts=0, accepted=0) for _ in self._parts]
+                    for i in range(len(t) - 1):
+                        self._run(pool, flat, [t[i], t[i + 1]], kwargs)
+                    raise
+            for i in range(len(t) - 1):
                 if callback:
                     callback(t[i])
-                span = [t[i], t[i + 1]] if callback else t
-                subs = [self._gather(flat, ranges) for _, _, ranges, _ in self._parts]
-                futs = [pool.submit(part.solve, sub, span, None, kwargs)
-                        for (part, _, _, _), sub in zip(self._parts, subs)]
-                try:
-                    for f in futs:
-                        f.result()
-                finally:  # a sub-batch that failed holds its last good interval's state
-                    wait(futs)
-                    for (_, _, ranges, _), sub in zip(self._parts, subs):
-                        self._scatter(flat, ranges, sub)
-                self._count_interval()
+                self._run(pool, flat, [t[i], t[i + 1]], kwargs)
         if callback and t:
             callback(t[-1])
+
+    def _run(self, pool, flat, span, kwargs):
+        """All sub-batches over the times of `span`; rho changes only if every one succeeds."""
+        subs = [self._gather(flat, ranges) for _, _, ranges, _ in self._parts]
+        futs = [pool.submit(part.solve, sub, span, None, kwargs) for (part, _, _, _), sub in zip(self._parts, subs)]
+        wait(futs)
+        for f in futs:
+            f.result()
+        for (_, _, ranges, _), sub in zip(self._parts, subs):
+            self._scatter(flat, ranges, sub)
+        self._count_interval()
 
     def _count_interval(self):
         # a sub-batch's counters restart with every solve (one interval, or all without a callback)
@@ -489,12 +502,11 @@ class batch_solver:
         t = [float(x) for x in t_list]
         self._counts = [dict(rhs=0, attempts=0, accepted=0) for _ in self._parts]
         with ThreadPoolExecutor(len(self._parts)) as pool:  # sub-batches run concurrently (own streams)
-            for i in range(len(t) - 1) if callback else range(min(1, len(t) - 1)):
+            for i in range(len(t) - 1):  # in place: joined at every output time, should a sub-batch fail
                 if callback:
                     callback(t[i])
-                span = [t[i], t[i + 1]] if callback else t
-                futs = [pool.submit(part.solve_device, int(rho_ptr) + 16 * ranges[0][0], span, None, kwargs)
-                        for part, _, ranges, _ in self._parts]
+                futs = [pool.submit(part.solve_device, int(rho_ptr) + 16 * ranges[0][0], [t[i], t[i + 1]], None,
+                                    kwargs) for part, _, ranges, _ in self._parts]
                 for f in futs:
                     f.result()
                 self._count_interval()

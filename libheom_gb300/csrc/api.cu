@@ -898,8 +898,12 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
       if (q->precision_eff == HEOMGB_FP64 && di.h_sym && n >= 4 && n <= 32) {
         std::vector<double> Hr(n2);
         for (int e = 0; e < n2; ++e) Hr[e] = H[e].real();
-        const std::vector<unsigned short> dig = split_h_digits(Hr.data(), n, &di.h_exp);
-        if (!dig.empty()) di.h_digits = reinterpret_cast<const uint4*>(q->arena.upload(dig, s));
+        std::vector<int> hx;
+        const std::vector<unsigned short> dig = split_h_digits(Hr.data(), n, hx);
+        if (!dig.empty()) {
+          di.h_digits = reinterpret_cast<const uint4*>(q->arena.upload(dig, s));
+          di.h_exp = q->arena.upload(hx, s);
+        }
       }
       if (rows_eligible(di, q->precision_eff == HEOMGB_MIXED)) {
         int4* rr = static_cast<int4*>(q->arena.alloc(sizeof(int4) * static_cast<size_t>(nh) * (1 + di.site_w)));

@@ -168,9 +168,9 @@ struct DiagInst {
   const double2* site_cm3_d;  // K * 3 and K * 2: the same coefficients in FP64 (the FP64 resident interval)
   const double2* site_cp2_d;
   const double2* site_cmn_d;  // site_cm3_d scaled by the occupation: row (3 k + case) * occ_rows + n_k
-  // k_rhs_split (FP64, real symmetric H): H's digits as its B operand, and the exponent of their scale
+  // k_rhs_split (FP64, real symmetric H): H's digits as its B operand, and the exponents of its columns' scales
   const uint4* h_digits;
-  int h_exp;
+  const int* h_exp;
 };
 struct DiagTile {
   int inst, l0, nt, pad;
@@ -306,7 +306,7 @@ bool sites_variant(int rows, int min_blocks, int block);  // a compiled (rows, C
 cudaError_t launch_site_records(const DiagInst& I, const int* msite, int4* rec, cudaStream_t s);
 // split.cu: H (n x n, row-major, real) as the digits of k_rhs_split's B operand (empty: out of range), whether an
 // instance can take the kernel, its ADOs per tile, threads and shared memory
-std::vector<unsigned short> split_h_digits(const double* H, int n, int* exponent);
+std::vector<unsigned short> split_h_digits(const double* H, int n, std::vector<int>& exponent);
 bool split_eligible(const DiagInst& I, bool mixed);
 int split_tile(int n);
 int split_threads();

@@ -4,52 +4,56 @@
 // stages).
 //
 // The FP64 pipe executes two operations per clock per SM, and 4 n of an
-// element's operations are the commutator.  Here rho and H are cut into seven
-// signed digits of nine bits each (fixed point, 62 bits below the largest
-// element of the ADO, or of H); the digits are integers of at most 256, exact
-// in FP16, and a product of two digit matrices summed over n <= 32 and over
-// the seven pairs of one order i + j stays below 2^24, so the FP32
-// accumulators of the tensor cores hold it exactly.  The orders 0 to 6 are
+// element's operations are the commutator.  Here rho and H are cut into eight
+// signed digits of nine bits each (fixed point, 70 bits below the largest value
+// of a row of rho's operand, or of a column of H); the digits are integers of at
+// most 256, exact in FP16, and a product of two digit matrices summed over
+// n <= 32 and over the eight pairs of one order i + j is at most 2^24, so the
+// FP32 accumulators of the tensor cores hold it exactly.  The orders 0 to 7 are
 // combined with integer operations and rounded to FP64 once per value; what is
-// left out (orders above 6 and bits of rho below 2^-62 of the ADO's largest)
-// is below 2^-57 of the largest product (the error-free splitting of matrix
-// products of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012).
-// Measured against extended precision over aggregates of 4 to 24 sites, states
-// after two steps: 1.34e-16 with either where the step leaves the state's own
-// rounding in charge, 4.0e-16 here and 4.7e-16 with the FP64 sums at 24 sites
-// where the operator is (steps 40 times longer).  A stage of the 24-site model
-// at depth 3 (12M elements) takes 0.59 ms, 2.95 with k_rhs_diag<double>, whose
-// FP64 pipe alone needs 2.58 (16 sites: 0.088 and 0.287).
+// left out (orders above 7 and bits of the values below 2^-70 of their row's
+// largest) is below n 2^-66.8 of the scale, the product of the row's and the
+// column's power of two (the error-free splitting of matrix products of Ozaki,
+// Ogita, Oishi and Rump, Numer. Algorithms 59, 2012).
 //
-// Per tile of T = 128 / (4 n) ADOs, the first group of a CTA (128 threads):
-//   1. the stage input (copied with cp.async a tile ahead), each ADO's largest
-//      exponent;
-//   2. digits of R, I, R^T and I^T (rho = R + iI; rows 4 n per ADO, K = n
-//      padded to 16) into the A operand, K-major without swizzle;
-//   3. MMAs (M = 128, one thread): digit i of rho against the digits 0..6-i of
-//      H at once (N = 7 - i blocks of n padded to 16), into the tensor-memory
-//      columns of the orders i..6, so 7 MMAs per 16 of K cover all 28 pairs;
+// Element by element the result is as good as FP64 sums, whose error is n 2^-53
+// of an element's own terms at worst: a component whose larger product reaches
+// 2^-13 of the scale has an error of n 2^-53.8 of it at worst (2^-55 in the mean),
+// and the others (2 in 10000 for 24 coupled sites, nearly all for a state
+// localised on a chain), rows whose largest value lies outside 2^-800 .. 2^900,
+// infinities and NaNs take FP64 sums in pass 5.  One scale for an ADO and seven
+// digits were faster (0.59 ms where this takes 0.78) and lost the small elements of
+// graded states.  Measured against 64 bits, four steps of 24 sites: 7.5e-17 of
+// the state's norm, as with FP64 sums.  A stage of the 24-site model at depth 3
+// (12M elements) takes 0.78 ms, 2.95 with k_rhs_diag<double>, whose FP64 pipe alone
+// needs 2.58 (16 sites: 0.115 and 0.287).
+//
+// Per tile of T = 128 / (4 n) ADOs, the first group of a CTA (256 threads):
+//   1. the stage input (copied with cp.async a tile ahead), the largest exponent
+//      of each row of R, I, R^T and I^T (rho = R + iI);
+//   2. the rows' digits (4 n rows per ADO, K = n padded to 16) into the A
+//      operand, K-major without swizzle;
+//   3. MMAs (M = 128, one thread): digit i of rho against the digits 0..7-i of
+//      H at once (N = 8 - i blocks of n padded to 16), into the tensor-memory
+//      columns of the orders i..7, so 8 MMAs per 16 of K cover all 36 pairs;
 //   4. read-back: rows of R H, I H (rho H) and R^T H, I^T H (H rho,
-//      transposed) as 64-bit integers in shared memory, in units of 2^-57 of the
-//      product of the largest elements (a sum of n <= 32 of them, and the
-//      difference of two sums, stay below 2^63);
-// and the second group (320 threads), a tile behind it:
-//   5. one element per thread: the difference of the two products, rounded to
-//      FP64 with integer operations; damping and +1 terms (ADOs below the
-//      deepest tier);
+//      transposed) in FP64 to shared memory;
+// and the second group (192 threads), a tile behind it:
+//   5. one element per thread: the difference of the two products, or FP64 sums
+//      (a few elements of a warp by the whole warp one after another, many lane
+//      by lane); damping and +1 terms (ADOs below the deepest tier);
 //   6. the -1 terms, one thread per element that a mode touches (an FP64
 //      instruction takes the pipe's 64 cycles whatever lanes it has: inside
 //      pass 5 these terms' few lanes made every warp pay, 0.44 of 1.22 ms);
 //   7. the stage epilogue, one element per thread.
 // The groups meet on named barriers: products full (first to second) and free
 // (second to first).  Two CTAs per SM, by tensor memory (256 of 512 columns)
-// and registers.  What bounds it now is the second group's chain: FP64 issue
-// (0.35 ms of the 0.59 a stage of 12M elements takes) and shared memory
-// latency; the first group alone takes 0.38.  Measured there: one group with
-// CTA barriers between the passes 0.86 ms; groups of 256 and 192 threads 0.69;
-// conversions and scaling on the FP64 pipe 0.69, the epilogue's loads ahead of
-// pass 5 0.63 (registers).  An ADO with elements beyond 2^900, infinities or
-// NaNs takes FP64 sums in pass 5.
+// and registers.  What bounds it: the first group's chain of integer work (digits,
+// read-back), then the second's FP64 issue and shared memory latency.  Measured at 24
+// sites, ms a stage: threads of the groups 128 and 320 0.89, 256 and 192 0.82, 256
+// and 224 0.84, 256 and 160 0.85, 384 and 128 1.07; the digits written four at a
+// time by row 0.79; pass 1 with two threads a row 0.78.  Without any FP64 sums
+// in pass 5 it would take 0.76, without pass 1 0.73.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -67,13 +71,19 @@ namespace heomgb {
 
 namespace {
 
-constexpr int kDigits = 7, kBits = 9;
-constexpr int kSplitX = 128, kSplitY = 320;  // threads of the two groups
+constexpr int kDigits = 8, kBits = 9;
+constexpr int kSplitX = 256, kSplitY = 192;  // threads of the two groups
 constexpr int kSplitThreads = kSplitX + kSplitY;
 constexpr int kBarX = 1, kBarY = 2, kBarFull = 3, kBarFree = 4;  // named barriers
-constexpr int kSplitCols = 256;  // tensor-memory columns of a CTA: seven orders of at most 32
-// the digits' bias: sum of 256 * 2^(9 k)
-constexpr unsigned long long kBias = 0x4020100804020100ull;
+constexpr int kSplitCols = 256;  // tensor-memory columns of a CTA: eight orders of at most 32
+// the bias of four digits: sum of 256 * 2^(9 k), k = 0..3
+constexpr unsigned long long kBias = 0x804020100ull;
+constexpr unsigned long long kLow = (1ull << 36) - 1;
+// A row's exponent field (s_exp): 0 for a row of zeros, kRowOut for one that the digits do not hold
+constexpr int kRowMin = 223, kRowMax = 1922, kRowOut = 3000;
+// A commutator's component whose larger product is below 2^-kTrust of its scale takes FP64 sums
+constexpr int kTrust = 13;
+constexpr int kNoColumn = -20000;  // the exponent of a column of zeros
 
 struct SplitGeom {
   int tile, rows, kp, np;  // ADOs; rows 4 n tile; K and N padded to 16
@@ -105,15 +115,24 @@ __host__ __device__ __forceinline__ size_t split_y_bytes(int n, int w) {
   return static_cast<size_t>(g.tile) * (n * n * sizeof(double2) + (1 + w) * sizeof(int4));
 }
 
-// |x| as a 62-bit fixed-point number below 2^61 at the scale of exponent es
-// (es >= the exponent field of x), with its sign
-__device__ __forceinline__ long long to_fixed(double x, int es) {
+// |x| truncated to 70 bits at the scale of the biased exponent es (at least x's), plus
+// the digits' bias: digits 0..3 in the low 36 bits of lo, 4..7 of hi
+struct Fixed {
+  unsigned long long lo, hi;
+  uint32_t sign;  // 0x8000 for a negative x
+};
+__device__ __forceinline__ Fixed to_fixed(double x, int es) {
   const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(x));
-  const int hi = static_cast<int>(u >> 32), ex = (hi >> 20) & 0x7ff;
-  const unsigned long long man = ex ? ((u & 0xfffffffffffffull) | (1ull << 52)) << 8 : 0ull;
-  const long long v = static_cast<long long>(man >> min(es - ex, 63));
-  const long long s = static_cast<long long>(hi >> 31);
-  return (v ^ s) - s;
+  const int ex = static_cast<int>(u >> 52) & 0x7ff;
+  const unsigned long long m = ex ? (u << 11) | (1ull << 63) : 0ull;  // the leading bit at 63: bit 69 of the 70
+  const int sh = min(es - ex, 97);
+  const unsigned long long hi = sh < 34 ? m >> (30 + sh) : 0ull;
+  const unsigned long long lo = (sh < 34 ? m << (34 - sh) : m >> (sh - 34)) >> 28;
+  Fixed f;
+  f.lo = lo + kBias;
+  f.hi = hi + kBias + (f.lo >> 36);
+  f.sign = static_cast<uint32_t>(u >> 48) & 0x8000u;
+  return f;
 }
 
 __device__ __forceinline__ uint32_t digit(unsigned long long y, int k) {  // the biased digit of weight 2^(9 k)
@@ -147,6 +166,15 @@ __device__ __forceinline__ double from_fixed(long long v, int e) {
   m = (m + 0x1ffull + ((m >> 10) & 1ull)) >> 10;  // 53 bits; a carry into bit 53 raises the exponent below
   const unsigned long long ex = static_cast<unsigned long long>(1023 + 62 - lz + e - 1);
   return __longlong_as_double(static_cast<long long>(s | ((ex << 52) + m)));
+}
+
+// sum of o[s] 2^(9 (7 - s)) over the eight orders, times 2^e, to the nearest double (|o| <= 2^24)
+__device__ __forceinline__ double from_orders(const int (&o)[kDigits], int e) {
+  const long long hi = mad_wide(o[0], 1 << 27, mad_wide(o[1], 1 << 18, mad_wide(o[2], 1 << 9, o[3])));
+  const long long lo = mad_wide(o[4], 1 << 27, mad_wide(o[5], 1 << 18, mad_wide(o[6], 1 << 9, o[7])));
+  // hi 2^36 + lo in the 62 bits from its leading one on
+  const int s = min(36, __clzll(hi < 0 ? -hi : hi) - 2);
+  return from_fixed((hi << s) + (lo >> (36 - s)), e + 36 - s);
 }
 
 // four columns of one order at taddr, without the wait
@@ -186,7 +214,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tslot;
-  __shared__ unsigned int s_max3[3][8];  // the largest exponents of a tile's ADOs, three tiles in turn
+  __shared__ short s_exp2[2][128];  // the exponent of every row of A, two tiles in turn
   __shared__ volatile int s_fail;  // 1 + the tile whose MMAs did not complete
   double dt;
   int cur;
@@ -195,14 +223,13 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
   const double2* __restrict__ y = stage_input<double2>(st, cur);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned char* As = smem_raw;
-  long long* P = reinterpret_cast<long long*>(smem_raw + ds.split_p);
+  double* P = reinterpret_cast<double*>(smem_raw + ds.split_p);
   unsigned char* Bs = smem_raw + ds.split_b;
   if (warp == 0) tmem_alloc(&tslot, kSplitCols);
   if (tid == 0) {
     mbar_init(&mbar);
     mbar_init_fence();
   }
-  if (tid < 24) s_max3[tid >> 3][tid & 7] = 0u;
   if (tid == 0) s_fail = 0;
   fence_before();
   __syncthreads();
@@ -213,44 +240,48 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
   if (tid < kSplitX) {
     // ---------------------------------------------------------------- first group: passes 1 to 4
     uint32_t parity = 0;
-    int b_inst = -1, buf = 0;
+    int b_inst = -1, buf = 0, eb = 0;
     DiagTile td{}, tdn{};
     if (blockIdx.x < ds.n_tiles) {
       tdn = ds.tiles[blockIdx.x];
       split_stage(ds.inst + tdn.inst, tdn, y, smem_raw + ds.split_y);
     }
-    for (int t = blockIdx.x; t < ds.n_tiles; t += step, buf = buf == 2 ? 0 : buf + 1) {
+    for (int t = blockIdx.x; t < ds.n_tiles; t += step, buf = buf == 2 ? 0 : buf + 1, eb ^= 1) {
       td = tdn;
       const DiagInst* __restrict__ I = ds.inst + td.inst;
       const int n = I->n, n2 = n * n;
       const SplitGeom g = split_geom(n);
-      const int nt = td.nt, ne = nt * n2;
+      const int nt = td.nt;
       const double2* ys = reinterpret_cast<const double2*>(smem_raw + ds.split_y + buf * ds.split_ybuf);
-      const float r_n2 = 1.0f / n2;
-      unsigned int* s_max = s_max3[buf];
-      // pass 1: the tile (in flight since the last one) has landed; a thread looks at what it copied
+      short* s_exp = s_exp2[eb];
+      // pass 1: the tile (in flight since the last one) has landed
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      {
-        unsigned int top = 0u;
-        int lt = 0;
-        for (int i = tid; i < ne; i += kSplitX) {
-          const double2 v = ys[i];
-          const unsigned int m = max(static_cast<unsigned int>(__double2hiint(v.x)) & 0x7fffffffu,
-                                     static_cast<unsigned int>(__double2hiint(v.y)) & 0x7fffffffu);
-          const int li = nt > 1 ? small_div(i, r_n2) : 0;
-          if (li != lt) {
-            atomicMax(&s_max[lt], top);
-            top = 0u;
-            lt = li;
+      bar_sync<kBarX, kSplitX>();
+      {  // two threads: a row of A, that is a row or a column of one component of an ADO
+        static_assert(kSplitX >= 256, "two threads for each of 128 rows");
+        const int row = tid >> 1;
+        unsigned int top = 0u, any = 0u;
+        if (row < nt * 4 * n) {
+          const float r_n = 1.0f / n;
+          const int q = small_div(row, r_n), lt = q >> 2, x = row - q * n;
+          const double* src = reinterpret_cast<const double*>(ys + lt * n2) + (q & 1);
+          const int ld = q & 2 ? n : 1, at = q & 2 ? x : x * n;
+          int c = x + (tid & 1);  // rows start at different columns: fewer bank conflicts
+          if (c >= n) c -= n;
+#pragma unroll 4
+          for (int i = 0; i < (n + 1) >> 1; ++i) {
+            const double v = src[2 * (at + c * ld)];
+            top = max(top, static_cast<unsigned int>(__double2hiint(v)) & 0x7fffffffu);
+            any |= static_cast<unsigned int>(__double2loint(v));
+            c += 2;
+            if (c >= n) c -= n;
           }
-          top = max(top, m);
         }
-        if (nt == 1) {
-          top = __reduce_max_sync(0xffffffffu, top);
-          if (lane == 0) atomicMax(&s_max[0], top);
-        } else {
-          atomicMax(&s_max[lt], top);
-        }
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        any |= __shfl_xor_sync(0xffffffffu, any, 1);
+        const int ex = static_cast<int>(top >> 20);
+        if ((tid & 1) == 0 && row < 128)
+          s_exp[row] = static_cast<short>((top | any) == 0u ? 0 : ex < kRowMin || ex > kRowMax ? kRowOut : ex);
       }
       const int n8 = (n + 7) & ~7;
       if (td.inst != b_inst) {  // H's digits, and the K padding of A
@@ -266,36 +297,30 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
         b_inst = td.inst;
       }
       bar_sync<kBarX, kSplitX>();
-      // pass 2: 2 x 2 blocks of one component, 16 of them an 8 x 8 block
+      // pass 2: four neighbours in K of a row of A per thread
       {
-        const int nb8 = n8 >> 3, per = 2 * nb8 * nb8 * 16;
-        const float r_per = 1.0f / per, r_nb = 1.0f / nb8;
+        const int rows = 4 * n, per = rows * (n8 >> 2);
+        const float r_per = 1.0f / per, r_rows = 1.0f / rows, r_n = 1.0f / n;
         for (int q = tid; q < nt * per; q += kSplitX) {
-          const int lt = small_div(q, r_per), r = q - lt * per, s16 = r & 15, sb = r >> 4;
-          const int comp = sb & 1, b8 = sb >> 1, A8 = small_div(b8, r_nb), C8 = b8 - A8 * nb8;
-          const int a = A8 * 8 + (s16 >> 2) * 2, c = C8 * 8 + (s16 & 3) * 2;
-          if (a >= n && c >= n) continue;
-          const int es = max(static_cast<int>(s_max[lt] >> 20), 223);
-          const double* src = reinterpret_cast<const double*>(ys + lt * n2) + comp;
-          unsigned long long v[4];
+          const int lt = small_div(q, r_per), r = q - lt * per, k4 = small_div(r, r_rows), row = r - k4 * rows;
+          const int m = lt * rows + row, part = small_div(row, r_n), x = row - part * n;
+          const double* src = reinterpret_cast<const double*>(ys + lt * n2) + (part & 1);
+          const int ld = part & 2 ? n : 1, at = part & 2 ? x : x * n;
+          const int es = min(static_cast<int>(s_exp[m]), 2047);
+          Fixed v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const int aj = a + (j >> 1), cj = c + (j & 1);
-            const double x = aj < n && cj < n ? src[2 * (aj * n + cj)] : 0.0;
-            v[j] = static_cast<unsigned long long>(to_fixed(x, es)) + kBias;
+            const int k = 4 * k4 + j;
+            v[j] = to_fixed(k < n ? src[2 * (at + k * ld)] : 0.0, es);
           }
-          const int m = lt * 4 * n + comp * n, mt = m + 2 * n;
-          auto at = [&](int row, int k) { return As + (row >> 3) * g.sbo + (k >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2; };
-          unsigned char *r0 = at(m + a, c), *r1 = at(m + a + 1, c), *t0 = at(mt + c, a), *t1 = at(mt + c + 1, a);
+          const uint32_t s0 = v[0].sign | (v[1].sign << 16), s1 = v[2].sign | (v[3].sign << 16);
+          unsigned char* to = As + (m >> 3) * g.sbo + (k4 >> 1) * 128 + (m & 7) * 16 + (k4 & 1) * 8;
 #pragma unroll
           for (int d = 0; d < kDigits; ++d) {
-            const int k = kDigits - 1 - d;
-            const uint32_t h0 = digit_pair(digit(v[0], k), digit(v[1], k)), h1 = digit_pair(digit(v[2], k), digit(v[3], k));
-            const int o = d * g.dstride;
-            if (a < n) *reinterpret_cast<uint32_t*>(r0 + o) = h0;
-            if (a + 1 < n) *reinterpret_cast<uint32_t*>(r1 + o) = h1;
-            if (c < n) *reinterpret_cast<uint32_t*>(t0 + o) = __byte_perm(h0, h1, 0x5410);
-            if (c + 1 < n) *reinterpret_cast<uint32_t*>(t1 + o) = __byte_perm(h0, h1, 0x7632);
+            const int w = kDigits - 1 - d;
+            auto dig = [&](const Fixed& f) { return w > 3 ? digit(f.hi, w - 4) : digit(f.lo, w); };
+            *reinterpret_cast<uint2*>(to + d * g.dstride) =
+                make_uint2(digit_pair(dig(v[0]), dig(v[1])) ^ s0, digit_pair(dig(v[2]), dig(v[3])) ^ s1);
           }
         }
       }
@@ -324,7 +349,6 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
       if (t != blockIdx.x) bar_sync<kBarFree, kSplitThreads>();  // the second group has read the last products
       // the second group is past the tile before the last one, whose buffer takes the next input
       const int nb = buf == 2 ? 0 : buf + 1;
-      if (t + step < ds.n_tiles && tid < 8) s_max3[nb][tid] = 0u;
       bar_sync<kBarX, kSplitX>();
       if (s_fail == t + 1) {
         bar_arrive<kBarFull, kSplitThreads>();  // the second group leaves too
@@ -339,6 +363,8 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
       // pass 4: warp w reads the lanes of sub-partition w % 4, in blocks of four columns
       if ((warp & 3) * 32 < nt * 4 * n) {
         const int m = (warp & 3) * 32 + lane;
+        // products of a row that the digits do not hold are not used
+        const int er = m < nt * 4 * n ? min(static_cast<int>(s_exp[m]), kRowMax) - 1022 - 77 : 0;
         for (int cb = warp >> 2; 4 * cb < n; cb += kSplitX / 128) {
           uint32_t f[kDigits][4];
 #pragma unroll
@@ -347,12 +373,11 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
+            if (m >= nt * 4 * n || cb * 4 + j >= n) continue;
             int o[kDigits];
 #pragma unroll
             for (int d = 0; d < kDigits; ++d) o[d] = __float2int_rn(__uint_as_float(f[d][j]));
-            const long long hi = mad_wide(o[0], 1 << 18, mad_wide(o[1], 1 << 9, o[2]));
-            const long long lo = mad_wide(o[3], 1 << 27, mad_wide(o[4], 1 << 18, mad_wide(o[5], 1 << 9, o[6])));
-            if (m < nt * 4 * n && cb * 4 + j < n) P[m * (n + 1) + cb * 4 + j] = (hi << 25) + ((lo + 1024) >> 11);
+            P[m * (n + 1) + cb * 4 + j] = from_orders(o, er + max(__ldg(I->h_exp + cb * 4 + j), -100));
           }
         }
       }
@@ -362,8 +387,8 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
   } else {
     // ---------------------------------------------------------------- second group: passes 5 to 7
     const int ty = tid - kSplitX;
-    int buf = 0;
-    for (int t = blockIdx.x; t < ds.n_tiles; t += step, buf = buf == 2 ? 0 : buf + 1) {
+    int buf = 0, eb = 0;
+    for (int t = blockIdx.x; t < ds.n_tiles; t += step, buf = buf == 2 ? 0 : buf + 1, eb ^= 1) {
       const DiagTile td = ds.tiles[t];
       const DiagInst* __restrict__ I = ds.inst + td.inst;
       const int n = I->n, n2 = n * n, K = I->K, w = I->site_w, w1 = 1 + w, void_idx = I->nh, tile = I->tile;
@@ -372,7 +397,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
       double2* ys = reinterpret_cast<double2*>(smem_raw + ds.split_y + buf * ds.split_ybuf);
       const int4* rec = reinterpret_cast<const int4*>(ys + static_cast<size_t>(tile) * n2);
       const float r_n2 = 1.0f / n2, r_n = 1.0f / n;
-      const unsigned int* s_max = s_max3[buf];
+      const short* s_exp = s_exp2[eb];
       bar_sync<kBarFull, kSplitThreads>();
       if (s_fail == t + 1) break;  // a later tile's failure does not concern this one
       // pass 5
@@ -400,29 +425,60 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_rhs_split(const DiagSet ds
       const int e_q = task(ty, lt_q, m_q);
       double2 v_q = make_double2(0.0, 0.0);
       if (e_q >= 0) v_q = __ldg(yi + static_cast<size_t>(rec[lt_q * w1 + 1 + m_q].y) * n2 + e_q);
-      for (int i = ty; i < ne; i += kSplitY) {
+      for (int ib = ty - lane; ib < ne; ib += kSplitY) {
+        const int i = min(ib + lane, ne - 1);
         const int lt = small_div(i, r_n2), e = i - lt * n2, a = small_div(e, r_n), b = e - a * n, l = l0 + lt;
-        const int ex = static_cast<int>(s_max[lt] >> 20), es = max(ex, 223);
         double2 acc;
-        if (ex <= 1922) {
-          const long long* Pl = P + lt * 4 * n * (n + 1);
-          const long long vx = Pl[(2 * n + b) * (n + 1) + a] - Pl[a * (n + 1) + b];
-          const long long vy = Pl[(3 * n + b) * (n + 1) + a] - Pl[(n + a) * (n + 1) + b];
-          const int u = es - 1022 + I->h_exp - 57;
-          acc.x = from_fixed(vx, u);
-          acc.y = from_fixed(vy, u);
-        } else {  // out of the fixed-point range
-          acc = make_double2(0.0, 0.0);
-          const double2* __restrict__ yl = yi + static_cast<size_t>(l) * n2;  // ys is being replaced
-          for (int c = 0; c < n; ++c) {
-            const double hac = I->H[a * n + c].x, hcb = I->H[c * n + b].x;
-            const double2 ycb = __ldg(yl + c * n + b), yac = __ldg(yl + a * n + c);
-            acc.x = fma(hac, ycb.x, acc.x);
-            acc.x = fma(-hcb, yac.x, acc.x);
-            acc.y = fma(hac, ycb.y, acc.y);
-            acc.y = fma(-hcb, yac.y, acc.y);
+        bool ok;
+        {
+          const int r0 = lt * 4 * n, ra = r0 + a, rb = r0 + 2 * n + b;
+          const double x2 = P[rb * (n + 1) + a], x1 = P[ra * (n + 1) + b];
+          const double y2 = P[(rb + n) * (n + 1) + a], y1 = P[(ra + n) * (n + 1) + b];
+          acc = make_double2(x2 - x1, y2 - y1);
+          const int ha = __ldg(I->h_exp + a), hb = __ldg(I->h_exp + b);
+          auto scale = [](int f) { return f == 0 ? kNoColumn : f == kRowOut ? 50000 : f - 1022; };
+          auto trusted = [&](double p2, double p1, int f2, int f1) {
+            const unsigned int top = max(static_cast<unsigned int>(__double2hiint(p2)) & 0x7fffffffu,
+                                         static_cast<unsigned int>(__double2hiint(p1)) & 0x7fffffffu);
+            return static_cast<int>(top >> 20) - 1023 + kTrust >= max(scale(f2) + ha, scale(f1) + hb);
+          };
+          ok = trusted(x2, x1, s_exp[rb], s_exp[ra]) && trusted(y2, y1, s_exp[rb + n], s_exp[ra + n]);
+        }
+        // FP64 sums of the others: lane by lane where there are many, else the warp on one after another
+        unsigned int rest = __ballot_sync(0xffffffffu, !ok && ib + lane < ne);
+        if (__popc(rest) * 4 > n) {
+          if (!ok) {
+            acc = make_double2(0.0, 0.0);
+            const double2* __restrict__ yl = yi + static_cast<size_t>(l) * n2;  // ys is being replaced
+            for (int c = 0; c < n; ++c) {
+              const double hac = I->H[a * n + c].x, hcb = I->H[c * n + b].x;
+              const double2 ycb = __ldg(yl + c * n + b), yac = __ldg(yl + a * n + c);
+              acc.x = fma(hac, ycb.x, acc.x);
+              acc.x = fma(-hcb, yac.x, acc.x);
+              acc.y = fma(hac, ycb.y, acc.y);
+              acc.y = fma(-hcb, yac.y, acc.y);
+            }
+          }
+        } else {
+          for (; rest; rest &= rest - 1) {
+            const int j = __ffs(rest) - 1, lj = small_div(ib + j, r_n2), ej = ib + j - lj * n2, aj = small_div(ej, r_n),
+                      bj = ej - aj * n;
+            double2 v = make_double2(0.0, 0.0);
+            if (lane < n) {
+              const double2* __restrict__ yl = yi + static_cast<size_t>(l0 + lj) * n2;
+              const double hac = I->H[aj * n + lane].x, hcb = I->H[lane * n + bj].x;
+              const double2 ycb = __ldg(yl + lane * n + bj), yac = __ldg(yl + aj * n + lane);
+              v.x = fma(-hcb, yac.x, hac * ycb.x);
+              v.y = fma(-hcb, yac.y, hac * ycb.y);
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+              v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+              v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+            }
+            if (lane == j) acc = v;
           }
         }
+        if (ib + lane >= ne) continue;
         double2 D = make_double2(-acc.y, acc.x);
         // damping
         const double2 d0 = __ldg(I->ngd + l), d1 = __ldg(I->c_sd + e), yv = ys[i];
@@ -508,24 +564,47 @@ SplitKernel split_kernel(int kind) {
 
 }  // namespace
 
-std::vector<unsigned short> split_h_digits(const double* H, int n, int* exponent) {
-  double top = 0.0;
+std::vector<unsigned short> split_h_digits(const double* H, int n, std::vector<int>& exponent) {
+  std::vector<double> top(n, 0.0);
+  double all = 0.0;
   for (int i = 0; i < n * n; ++i) {
     if (!std::isfinite(H[i])) return {};
-    top = std::max(top, std::fabs(H[i]));
+    top[i % n] = std::max(top[i % n], std::fabs(H[i]));
+    all = std::max(all, std::fabs(H[i]));
   }
   int eh = 0;
-  if (top > 0.0) std::frexp(top, &eh);  // top < 2^eh
+  if (all > 0.0) std::frexp(all, &eh);  // all < 2^eh
   if (eh < -100 || eh > 100) return {};
-  *exponent = eh;
+  exponent.assign(n, kNoColumn);
+  for (int b = 0; b < n; ++b)
+    if (top[b] > 0.0) {
+      std::frexp(top[b], &exponent[b]);
+      exponent[b] = std::max(exponent[b], -100);
+    }
   const SplitGeom g = split_geom(n);
   std::vector<unsigned short> out(split_b_bytes(n) / 2, 0);
   for (int b = 0; b < n; ++b)
     for (int c = 0; c < n; ++c) {
-      unsigned long long v =
-          static_cast<unsigned long long>(static_cast<long long>(std::ldexp(H[c * n + b], 61 - eh))) + kBias;
+      // |H| truncated to 70 bits below the column's power of two, as to_fixed does
+      int ex = 0;
+      const double frac = std::frexp(std::fabs(H[c * n + b]), &ex);
+      if (frac == 0.0) continue;
+      const unsigned long long man = static_cast<unsigned long long>(std::ldexp(frac, 53));
+      const int sh = 17 + ex - exponent[b];  // at most 17
+      unsigned long long hi = 0, lo = 0;
+      if (sh > 0) {
+        hi = man >> (36 - sh);
+        lo = (man << sh) & kLow;
+      } else if (sh > -53) {
+        hi = (man >> -sh) >> 36;
+        lo = (man >> -sh) & kLow;
+      }
+      lo += kBias;
+      hi += kBias + (lo >> 36);
       for (int d = 0; d < kDigits; ++d) {
-        const int dig = static_cast<int>((v >> (kBits * (kDigits - 1 - d))) & 0x1ff) - 256;
+        const int w = kDigits - 1 - d;
+        int dig = static_cast<int>((w > 3 ? hi >> (kBits * (w - 4)) : lo >> (kBits * w)) & 0x1ff) - 256;
+        if (H[c * n + b] < 0.0) dig = -dig;
         // the digit's FP16 bits: sign, exponent, ten fraction bits
         unsigned short h = 0;
         if (dig != 0) {

@@ -233,8 +233,8 @@ heomgb_status heomgb_qme_solver_resident(const heomgb_qme_solver* qs, int* on, i
 heomgb_status heomgb_qme_solver_row_kernel(const heomgb_qme_solver* qs, int* on);
 /* 1 when the solver's FP64 stages compute the commutator on the tensor cores
  * from exact digits (site-local baths, real symmetric H, 4 to 32 levels).
- * HEOMGB_SPLIT=0 keeps it out of the search, =1 takes it before the FP64
- * kernel.  No reference counterpart. */
+ * Taken by a rule on sizes; HEOMGB_SPLIT=0 keeps it out, =1 takes it wherever it
+ * can run.  No reference counterpart. */
 heomgb_status heomgb_qme_solver_split(const heomgb_qme_solver* qs, int* on);
 /* Whether fixed steps run as cluster-resident intervals (one launch per output
  * interval, a thread-block cluster of `size` CTAs of `block` threads per bin of

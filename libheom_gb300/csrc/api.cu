@@ -1635,15 +1635,14 @@ void autotune(heomgb_qme_solver* qs) {
         }
       }
   }
-  // FP64: the commutator on the tensor cores where every instance is eligible;
-  // HEOMGB_SPLIT=0 keeps it out, =1 keeps k_rhs_diag out
-  bool split_ok = !insts.empty(), split_only = false, best_split = false;
+  // FP64: the commutator on the tensor cores, by a rule on sizes and not by the
+  // search: its roundings are not k_rhs_diag's, and the same model has to give the same
+  // bits in every run.  HEOMGB_SPLIT=0 keeps it out, =1 takes it wherever it can run
+  bool split_ok = !insts.empty(), best_split = false;
   for (const DiagInst& I : insts) split_ok = split_ok && split_eligible(I, qs->mixed);
-  if (const char* env = std::getenv("HEOMGB_SPLIT")) {
-    if (std::string(env) == "0") split_ok = false;
-    split_only = split_ok && std::string(env) == "1";
-  }
-  if (split_ok && !pin_b) {
+  const char* split_env = std::getenv("HEOMGB_SPLIT");
+  split_ok = split_ok && (split_env ? std::string(split_env) == "1" : split_pays(insts));
+  if (split_ok && !pin_b && !pin_tc && !pin_sb) {
     try {
       build_split_plan(qs->plan, insts, q->n_sm, qs->stream);
       const float ms = time_plan(split_threads());
@@ -1653,10 +1652,8 @@ void autotune(heomgb_qme_solver* qs) {
       ck(cudaStreamSynchronize(qs->stream), "ctl sync");
       if (probe.status == 2) {
         ck(cudaMemsetAsync(&qs->ctl->status, 0, sizeof(int), qs->stream), "ctl reset");
-      } else if (const float cost = ms * (qs->kind == HEOMGB_RKDP ? 1.15f : 1.f); cost < best) {
-        // Dormand-Prince: the timed stage's epilogue is a middling one, and the longer ones weigh
-        // more here (7 sites, depth 4: 31 us timed, 41 on average; k_rhs_diag 33 and 38)
-        best = cost;
+      } else {
+        best = ms;
         best_split = true;
       }
     } catch (const unsupported_error&) {
@@ -1668,7 +1665,7 @@ void autotune(heomgb_qme_solver* qs) {
     for (int e : epts)
       for (int mi = 0; mi < n_minb; ++mi) {
       const int m = minbs[mi];
-      if (pin_tc || pin_sb || (rows_only && best_rows) || (split_only && best_split) || (pin_b && (b != pin_b || e != pin_e || m != pin_m))) continue;
+      if (pin_tc || pin_sb || (rows_only && best_rows) || best_split || (pin_b && (b != pin_b || e != pin_e || m != pin_m))) continue;
       try {
         build_plan(qs->plan, insts, b, e, m, qs->mixed, q->n_sm, qs->stream);
       } catch (const unsupported_error&) {
@@ -1687,7 +1684,7 @@ void autotune(heomgb_qme_solver* qs) {
         best_b = b;
         best_e = e;
         best_m = m;
-        best_tc = best_sites = best_rows = best_split = false;
+        best_tc = best_sites = best_rows = false;
       }
     }
   cudaEventDestroy(e0);
@@ -1977,7 +1974,7 @@ void plan_local(heomgb_qme_solver* qs) {
 void plan_cluster(heomgb_qme_solver* qs) {
   const NvtxRange range("heomgb plan: cluster-resident bins");
   qs->cluster = false;
-  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || qs->path != PATH_DIAG || qs->term) return;
+  if ((qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4) || qs->path != PATH_DIAG || qs->term || qs->plan.split) return;
   bool force = false;
   if (const char* env = std::getenv("HEOMGB_CLUSTER")) {
     if (std::string(env) == "0") return;

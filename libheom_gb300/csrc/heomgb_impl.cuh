@@ -305,9 +305,10 @@ size_t sites_smem(int n, int K, int tile, int w);
 bool sites_variant(int rows, int min_blocks, int block);  // a compiled (rows, CTAs per SM, CTA size) variant
 cudaError_t launch_site_records(const DiagInst& I, const int* msite, int4* rec, cudaStream_t s);
 // split.cu: H (n x n, row-major, real) as the digits of k_rhs_split's B operand (empty: out of range), whether an
-// instance can take the kernel, its ADOs per tile, threads and shared memory
+// instance can take the kernel and whether a set of them is faster with it, its ADOs per tile, threads and shared memory
 std::vector<unsigned short> split_h_digits(const double* H, int n, std::vector<int>& exponent);
 bool split_eligible(const DiagInst& I, bool mixed);
+bool split_pays(const std::vector<DiagInst>& insts);
 int split_tile(int n);
 int split_threads();
 void split_smem(const DiagInst& I, size_t* a, size_t* p, size_t* b, size_t* y);

@@ -625,6 +625,24 @@ bool split_eligible(const DiagInst& I, bool mixed) {
          I.max_terms <= 4;
 }
 
+// Where the kernel beats k_rhs_diag<double>: the commutator's share of an element
+// grows with n, and a tile's chain of passes has to be hidden behind other tiles.
+// Measured, us a stage of k_rhs_diag<double> and of this, LSRK4 (RK4 alike): 8
+// levels, 310k elements 47 and 49; 10, 23k 10 and 17, 177k 34 and 26; 12, 47k 19 and 18
+// (Dormand-Prince 25 and 26), 421k 73 and 45; 13, 64k 19 and 19; 16, 144k 35 and 24; 24, 28k
+// 32 and 26, 12M 2944 and 783; 32, 67k 55 and 37.
+bool split_pays(const std::vector<DiagInst>& insts) {
+  long long elems = 0, work = 0;
+  int n = 32;
+  for (const DiagInst& I : insts) {
+    const long long e = static_cast<long long>(I.n2) * I.nh;
+    elems += e;
+    work += e * I.n;
+    n = std::min(n, I.n);
+  }
+  return n >= 10 && elems >= 25000 && work >= (n >= 16 ? 600000 : 1500000);
+}
+
 int split_tile(int n) { return split_geom(n).tile; }
 
 void split_smem(const DiagInst& I, size_t* a, size_t* p, size_t* b, size_t* y) {

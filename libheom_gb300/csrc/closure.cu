@@ -847,7 +847,7 @@ cudaError_t launch_term_fused(TermMlpArgs a, int n_sm, bool y_float, cudaStream_
   const int grid = (a.n_tier + a.apt - 1) / a.apt;
   const void* kern = y_float ? reinterpret_cast<const void*>(k_term_mlp<float2>)
                              : reinterpret_cast<const void*>(k_term_mlp<double2>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(kern);
   if (e != cudaSuccess) return e;
   if (y_float)
     k_term_mlp<float2><<<grid, kThrAll, smem, s>>>(a);
@@ -863,9 +863,9 @@ size_t train_image_bytes(int din, int h, int dout, int tiles) { return TrainImag
 cudaError_t launch_train(const TrainArgs& a, cudaStream_t s) {
   const size_t smem = train_smem_bytes(a.din, a.h, a.dout);
   const int tiles = train_tiles(a.B);
-  cudaError_t e = cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_train));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDwSmem));
+  e = allow_smem(reinterpret_cast<const void*>(k_dw));
   if (e != cudaSuccess) return e;
   k_train<<<tiles, kThrAll, smem, s>>>(a);
   int n = 0;

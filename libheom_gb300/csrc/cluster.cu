@@ -419,11 +419,8 @@ const void* cluster_kernel(bool mixed, int scheme, int ept) {
 
 cudaError_t configure(const void* kern, int size, size_t smem, int grid, int block, cudaStream_t s,
                       cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e == cudaSuccess && size > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   // the largest shared-memory split, so that the launches of two sub-batches can share an SM
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  const cudaError_t e = allow_smem(kern, true, true);
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = size;
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;

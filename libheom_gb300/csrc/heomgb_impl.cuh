@@ -283,6 +283,11 @@ int cluster_active(bool mixed, int scheme, int ept, int size, int block, size_t 
 cudaError_t launch_cluster(const ClusterArgs& args, bool mixed, int scheme, int ept, int size, int bins, int block,
                            size_t smem, cudaStream_t s);
 
+// Lifts a kernel's limits to the device's: dynamic shared memory, and (largest) the
+// shared-memory split, (wide) clusters of 16.  Once per kernel and device and
+// never lowered: solvers on other host threads launch the same kernel with
+// sizes of their own.
+cudaError_t allow_smem(const void* kern, bool largest = false, bool wide = false);
 // Launchers (kernels.cu).  `mixed` selects FP32 bulk arithmetic; `in_double`
 // says the RHS input is a double2 array even in mixed mode.  `ds` describes
 // the diagonal-coupling work (PATH_DIAG only).

@@ -8,7 +8,10 @@
 
 #include <cmath>
 #include <cstdint>
+#include <mutex>
+#include <set>
 #include <type_traits>
+#include <utility>
 
 #include "heomgb_impl.cuh"
 #include "fpconv.cuh"
@@ -1417,9 +1420,7 @@ static const void* resident_kernel(int scheme, bool hreal, int ept, int n) {
 
 int resident_blocks_per_sm(int scheme, bool hreal, int ept, int n, int block, size_t smem) {
   const void* kern = resident_kernel(scheme, hreal, ept, n);
-  if (!kern) return 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return 0;
+  if (!kern || allow_smem(kern) != cudaSuccess) return 0;
   int nb = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, block, smem) != cudaSuccess) return 0;
   return nb;
@@ -1429,7 +1430,7 @@ cudaError_t launch_resident(const ResidentArgs& args, int scheme, bool hreal, in
                             size_t smem, cudaStream_t s) {
   const void* kern = resident_kernel(scheme, hreal, ept, args.inst.n);
   if (!kern) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(kern);
   if (e != cudaSuccess) return e;
   ResidentArgs a = args;
   void* params[] = {&a};
@@ -1707,13 +1708,9 @@ static const void* local_kernel(bool mixed, int scheme) {
 
 int local_blocks_per_sm(bool mixed, int scheme, int block, size_t smem) {
   const void* kern = local_kernel(mixed, scheme);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return 0;
   // every instance takes the largest shared-memory split, so that the FP64 and the mixed
   // sub-batch's bins (different sizes) can share an SM
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) !=
-      cudaSuccess)
-    return 0;
+  if (allow_smem(kern, true) != cudaSuccess) return 0;
   int nb = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, block, smem) != cudaSuccess) return 0;
   return nb;
@@ -1722,9 +1719,7 @@ int local_blocks_per_sm(bool mixed, int scheme, int block, size_t smem) {
 cudaError_t launch_local(const LocalArgs& args, bool mixed, int scheme, int grid, int block, size_t smem,
                          cudaStream_t s) {
   const void* kern = local_kernel(mixed, scheme);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  cudaError_t e = allow_smem(kern, true);
   if (e != cudaSuccess) return e;
   LocalArgs a = args;
   void* params[] = {&a};
@@ -2016,6 +2011,28 @@ __global__ void __launch_bounds__(256) k_rhs_redfield(const RhsModel m, const St
 }
 
 // ------------------------------------------------------------------ launch configuration
+cudaError_t allow_smem(const void* kern, bool largest, bool wide) {
+  static std::mutex lock;
+  static std::set<std::pair<const void*, int>> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> hold(lock);
+  if (done.count({kern, dev})) return cudaSuccess;
+  cudaFuncAttributes fa;
+  int top = 0;
+  e = cudaFuncGetAttributes(&fa, kern);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&top, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             top - static_cast<int>(fa.sharedSizeBytes));
+  if (e == cudaSuccess && largest)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess && wide) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) done.insert({kern, dev});
+  return e;
+}
+
 int rhs_block_size(const RhsModel& m, int path) {
   if (path != PATH_DIAG) {
     // k_rhs_liou forms all its baths' Phi and Psi together
@@ -2087,28 +2104,25 @@ static cudaError_t launch_typed(const RhsModel& m, const DiagSet* ds, const Stag
       if (ds->tcore) kern = ds->min_blocks == 3 ? k_rhs_diag_tc<TB, 3> : k_rhs_diag_tc<TB, 2>;
     }
     if (dsm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dsm));
+      cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern));
       if (e != cudaSuccess) return e;
     }
     kern<<<grid, block, dsm, s>>>(*ds, st);
   } else if (path == PATH_GENERAL) {
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k_rhs_general<TC, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
+      cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_rhs_general<TC, TB>));
       if (e != cudaSuccess) return e;
     }
     k_rhs_general<TC, TB><<<grid, block, smem, s>>>(m, st);
   } else if (path == PATH_REDFIELD) {
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k_rhs_redfield<TC, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
+      cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_rhs_redfield<TC, TB>));
       if (e != cudaSuccess) return e;
     }
     k_rhs_redfield<TC, TB><<<1, block, smem, s>>>(m, st);
   } else {
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k_rhs_liou<TC, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
+      cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_rhs_liou<TC, TB>));
       if (e != cudaSuccess) return e;
     }
     k_rhs_liou<TC, TB><<<grid, block, smem, s>>>(m, st);
@@ -2352,7 +2366,7 @@ cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, int
   const int n2 = n * n, per = std::max(1, 256 / n2);
   const size_t smem = sizeof(double2) * static_cast<size_t>(n2) * (1 + 2 * per);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_rotate, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_rotate));
     if (e != cudaSuccess) return e;
   }
   const int grid = static_cast<int>(std::min<long long>((count + per - 1) / per, 152 * 8));

@@ -449,7 +449,7 @@ size_t rows_warp(const DiagInst& I, int ados) {
 int rows_resident(const DiagSet& ds, int kind, int block) {
   RowsKernel kern = rows_kernel(ds, kind);
   if (ds.smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ds.smem)) != cudaSuccess)
+      allow_smem(reinterpret_cast<const void*>(kern)) != cudaSuccess)
     return 0;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, ds.smem) != cudaSuccess) return 0;
@@ -460,7 +460,7 @@ cudaError_t launch_rows(const DiagSet& ds, const Stage& st, int grid, int block,
   if (st.kind == EPI_DIFF) return cudaErrorInvalidValue;  // calc_diff keeps k_rhs_diag
   RowsKernel kern = rows_kernel(ds, st.kind);
   if (ds.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ds.smem));
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern));
     if (e != cudaSuccess) return e;
   }
   kern<<<grid, block, ds.smem, s>>>(ds, st);

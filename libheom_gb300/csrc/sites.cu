@@ -418,7 +418,7 @@ cudaError_t launch_kind(const DiagSet& ds, const Stage& st, int grid, int block,
   else
     kern = k_rhs_sites<KIND, 2, 384, 2>;
   if (ds.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ds.smem));
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern));
     if (e != cudaSuccess) return e;
   }
   kern<<<grid, block, ds.smem, s>>>(ds, st);

@@ -657,7 +657,7 @@ int split_threads() { return kSplitThreads; }
 cudaError_t launch_split(const DiagSet& ds, const Stage& st, int grid, cudaStream_t s) {
   SplitKernel kern = split_kernel(st.kind);
   if (!kern) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ds.smem));
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern));
   if (e != cudaSuccess) return e;
   kern<<<grid, kSplitThreads, ds.smem, s>>>(ds, st);
   ++g_launches;

@@ -193,7 +193,7 @@ cudaError_t launch_gemm_bf16(GemmArgs g, cudaStream_t s) {
   while (cols < g.bn) cols *= 2;
   g.tmem_cols = cols;
   const size_t smem = gemm_smem(g.bn);
-  cudaError_t e = cudaFuncSetAttribute(k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_gemm_bf16));
   if (e != cudaSuccess) return e;
   const dim3 grid((g.M + kBM - 1) / kBM, (g.N + g.bn - 1) / g.bn);
   k_gemm_bf16<<<grid, kThreads, smem, s>>>(g);

@@ -12,6 +12,7 @@
 #include <limits>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -19,6 +20,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "heomgb.h"
+#include "eigenbasis.h"
 #include "heomgb_impl.cuh"
 
 // NVTX ranges around the host-side phases (model set-up, planning and tile
@@ -445,6 +447,11 @@ struct heomgb_qme {
   // fixed-step solves, and the basis (null: none)
   DiagInst rinst{};
   const double2* rbasis = nullptr;
+  const double2* rbasis_lo = nullptr;  // what rbasis leaves out
+  bool rot_known = true;               // rotated_model has answered
+  std::mutex rot_lock;
+  std::vector<int> bath_ptr_h;         // what it needs of the model
+  std::vector<cd> sigma_h, sv_h, av_h;
   DiagPlan diff_plan;        // tiles for calc_diff
   heomgb_mlp* term = nullptr;  // learned terminator (not owned); null = plain truncation
   const float2* term_cke = nullptr;  // its set-up tables (TermModel::cke, sgn), in term_arena
@@ -916,47 +923,44 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
   return di;
 }
 
-// A basis in which every V_u is diagonal: W with W^dagger V_u W = diag(vd[u]),
-// where the V_u are Hermitian and commute (one bath always does).  The
-// eigenvectors of a fixed combination of them, checked on each; eigenvalues
-// that agree to rounding are made equal, so that no term hangs on their
-// difference.
-bool common_basis(const heomgb_qme* q, std::vector<cd>& W, std::vector<std::vector<cd>>& vd) {
+// The model's instance in the common eigenbasis of its V_u, where they have one
+// (a single bath always does), for the fixed-step solvers that work there;
+// false: none.  Formed when the first of them asks for it.
+bool rotated_model(heomgb_qme* q) {
+  std::lock_guard<std::mutex> hold(q->rot_lock);
+  if (q->rot_known) return q->rbasis != nullptr;
+  q->rot_known = true;
   const int n = q->n, n2 = n * n;
-  std::vector<cd> M(n2, cd(0.0, 0.0));
-  std::vector<double> top(q->U, 0.0);
+  if (n > kRotateMaxN || q->U == 0 || diag_tile_smem(n2, q->K, 1, false) > 200 * 1024) return false;
+  // the eigenvectors of a fixed combination of the V_u, checked on each
+  std::vector<cd> M(n2, cd(0.0, 0.0)), W0;
+  std::vector<std::vector<cd>> V(q->U), vd;
   double w = 1.0;
   for (int u = 0; u < q->U; ++u, w *= 0.618033988749895) {
-    const std::vector<cd>& V = q->baths[u].V;
-    for (const cd& v : V) top[u] = std::max(top[u], std::abs(v));
-    if (!(top[u] > 0.0) || !std::isfinite(top[u])) return false;
-    for (int a = 0; a < n; ++a)
-      for (int b = 0; b < n; ++b) {
-        if (std::abs(V[a * n + b] - std::conj(V[b * n + a])) > 1e-15 * top[u]) return false;
-        M[a * n + b] += w / top[u] * V[a * n + b];
-      }
+    V[u] = q->baths[u].V;
+    if (!plain_hermitian(V[u], n)) return false;
+    double top = 0.0;
+    for (const cd& v : V[u]) top = std::max(top, std::abs(v));
+    for (int e = 0; e < n2; ++e) M[e] += w / top * V[u][e];
   }
   std::vector<double> ev;
-  hermitian_eigen(M, n, ev, W);
-  vd.assign(q->U, std::vector<cd>(n));
-  for (int u = 0; u < q->U; ++u) {
-    const std::vector<cd>& V = q->baths[u].V;
-    for (int i = 0; i < n; ++i)
-      for (int j = 0; j < n; ++j) {
-        cd acc(0.0, 0.0);
-        for (int a = 0; a < n; ++a)
-          for (int b = 0; b < n; ++b) acc += std::conj(W[a * n + i]) * V[a * n + b] * W[b * n + j];
-        if (i == j)
-          vd[u][i] = cd(acc.real(), 0.0);
-        else if (std::abs(acc) > 1e-14 * top[u])
-          return false;
-      }
-    for (int i = 0; i < n; ++i) {
-      if (std::abs(vd[u][i]) <= 1e-14 * top[u]) vd[u][i] = cd(0.0, 0.0);
-      for (int j = 0; j < i; ++j)
-        if (std::abs(vd[u][i] - vd[u][j]) <= 1e-14 * top[u]) vd[u][i] = vd[u][j];
-    }
+  hermitian_eigen(M, n, ev, W0);
+  MatrixC W = twofold(W0);
+  if (!common_eigenbasis(V, M, n, W, vd)) return false;
+  const MatrixC H2 = in_basis(twofold(q->H), W, n);
+  std::vector<cd> H(n2), hi(n2), lo(n2);
+  for (int e = 0; e < n2; ++e) {
+    H[e] = H2[e].hi();
+    hi[e] = W[e].hi();
+    lo[e] = W[e].lo();
+    if (!std::isfinite(H[e].real()) || !std::isfinite(H[e].imag())) return false;
   }
+  cudaStream_t s = q->stream();
+  q->rinst = make_diag_inst(q, H, vd, q->bath_ptr_h, q->sigma_h, q->sv_h, q->av_h, s);
+  const double2* dhi = q->arena.upload(to_d2(hi), s);
+  q->rbasis_lo = q->arena.upload(to_d2(lo), s);
+  ck(cudaStreamSynchronize(s), "basis upload");
+  q->rbasis = dhi;
   return true;
 }
 
@@ -972,7 +976,8 @@ void build_model(heomgb_qme* q) {
   q->term = nullptr;  // a rebuilt model starts with plain truncation
   q->diff_tb = TermBuffers{};
   q->ready = false;
-  q->rbasis = nullptr;
+  q->rbasis = q->rbasis_lo = nullptr;
+  q->rot_known = true;  // no basis, unless the form below may have one
   cudaStream_t s = q->stream();
   const int n = q->n, n2 = n * n, U = q->U;
   // linear mode index lk (heom.h:65-74) and per-mode coefficients
@@ -1149,25 +1154,15 @@ void build_model(heomgb_qme* q) {
     if (rhs_smem_bytes(m, PATH_GENERAL, false) > 200 * 1024)
       throw unsupported_error("general-V Hilbert path supports n_level <= 50");
     // FP64 models whose V_u share an eigenbasis: fixed-step solves (linear in the
-    // state, so a change of basis commutes with them) run there on the
-    // diagonal-coupling kernels, which drop the n-term products of every bath
-    // and reach the resident plans (two levels, V = sigma_x, depth 10: 9.7 us a
-    // stage in k_rhs_general, 2.1 in the basis; the state's way in and out adds
-    // one k_rotate each).  The mixed form stays: its FP32 rounding depends on
-    // the basis.
-    std::vector<cd> W;
-    std::vector<std::vector<cd>> vd;
-    if (q->precision_eff == HEOMGB_FP64 && U > 0 && common_basis(q, W, vd) &&
-        diag_tile_smem(n2, K, 1, false) <= 200 * 1024) {
-      std::vector<cd> Hr(n2, cd(0.0, 0.0)), T(n2, cd(0.0, 0.0));
-      for (int a = 0; a < n; ++a)
-        for (int b = 0; b < n; ++b)
-          for (int j = 0; j < n; ++j) T[a * n + j] += q->H[a * n + b] * W[b * n + j];
-      for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j)
-          for (int a = 0; a < n; ++a) Hr[i * n + j] += std::conj(W[a * n + i]) * T[a * n + j];
-      q->rinst = make_diag_inst(q, Hr, vd, bath_ptr, sigma, sv, av, s);
-      q->rbasis = q->arena.upload(to_d2(W), s);
+    // state, so a change of basis commutes with them) run there as cluster-resident
+    // intervals where the model fits a cluster (plan_rotated).  The mixed form
+    // stays: its FP32 rounding depends on the basis.
+    if (q->precision_eff == HEOMGB_FP64) {
+      q->rot_known = false;
+      q->bath_ptr_h = bath_ptr;
+      q->sigma_h = sigma;
+      q->sv_h = sv;
+      q->av_h = av;
     }
   } else if (q->path == PATH_LIOU) {
     // superoperators (heom_liou.h:71-99)
@@ -1320,6 +1315,7 @@ void autotune(heomgb_qme_solver* qs);
 void plan_resident(heomgb_qme_solver* qs);
 void plan_local(heomgb_qme_solver* qs);
 void plan_cluster(heomgb_qme_solver* qs);
+bool plan_rotated(heomgb_qme_solver* qs);
 
 // The model's instance in the basis that the solver works in.
 const DiagInst& solver_inst(const heomgb_qme_solver* qs) { return qs->rotated ? qs->q->rinst : qs->q->dinst; }
@@ -1391,8 +1387,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
   for (heomgb_qme* m : qs->qmes) N += m->main_size();
   qs->N = N;
   qs->mixed = q->precision_eff == HEOMGB_MIXED;
-  qs->rotated = q->rbasis && qs->kind != HEOMGB_RKDP;  // the error norm is not invariant
-  qs->path = qs->rotated ? PATH_DIAG : q->path;
+  qs->path = q->path;
   qs->col_major = q->col_major != 0;
   qs->separate = qs->mixed;
   const size_t bd = sizeof(double2) * N;
@@ -1408,7 +1403,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
     qs->Ytmp[1] = A.alloc(bb);
   }
   if (qs->kind == HEOMGB_RK4 || qs->kind == HEOMGB_LSRK4) qs->acc = static_cast<double2*>(A.alloc(bd));
-  if (qs->col_major || qs->rotated) qs->otmp = static_cast<double2*>(A.alloc(bd));
+  if (qs->col_major) qs->otmp = static_cast<double2*>(A.alloc(bd));
   if (qs->kind == HEOMGB_RKDP)
     for (int i = 0; i < 6; ++i) qs->K[i] = A.alloc(bb);
   qs->ctl = static_cast<DpCtl*>(A.alloc(sizeof(DpCtl)));
@@ -1421,6 +1416,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
     if (qs->qmes.size() != 1) throw unsupported_error("the learned terminator is not available in batches");
     alloc_term(qs->arena, q, qs->tb);
   }
+  if (plan_rotated(qs)) return;
   // a model that runs as resident intervals needs no tile search: its stage
   // kernels (the fall-back, should the device not hold the cooperative grid) take
   // the default shape
@@ -1440,6 +1436,34 @@ void alloc_solver(heomgb_qme_solver* qs) {
   if (std::getenv("HEOMGB_TILE")) plan_resident(qs);
   plan_local(qs);
   plan_cluster(qs);
+}
+
+// Fixed steps of a dense FP64 model in the common eigenbasis of its V_u
+// (rotated_model): cluster-resident intervals with compensated state sums, where
+// the model fits a cluster; no other plan is looked for, since the products of
+// every bath drop out there (two levels, V = sigma_x, depth 10: 9.7 us a stage in
+// k_rhs_general, 2.1 in the basis) and the plain kernels would add the
+// rounding of the way in and out.  Dormand-Prince stays: its error norm is
+// not invariant.  HEOMGB_CLUSTER=0, and every pinned plan, keeps k_rhs_general.
+bool plan_rotated(heomgb_qme_solver* qs) {
+  heomgb_qme* q = qs->q;
+  if (q->path != PATH_GENERAL || qs->mixed || qs->qmes.size() != 1 || (qs->kind != HEOMGB_RK4 && qs->kind != HEOMGB_LSRK4))
+    return false;
+  if (!rotated_model(q)) return false;
+  qs->rotated = true;
+  qs->path = PATH_DIAG;
+  build_plan(qs->plan, solver_instances(qs), 128, 4, 1, false, q->n_sm, qs->stream);
+  qs->block = qs->plan.block;
+  qs->grid = qs->plan.grid;
+  plan_cluster(qs);
+  if (!qs->cluster) {
+    qs->rotated = false;
+    qs->path = q->path;
+    return false;
+  }
+  qs->partials = static_cast<double*>(qs->arena.alloc(sizeof(double) * std::max(qs->grid, 1)));
+  qs->otmp = qs->otmp ? qs->otmp : static_cast<double2*>(qs->arena.alloc(sizeof(double2) * qs->N));
+  return true;
 }
 
 // Tile shape search for the diagonal-coupling kernel: CTA size x elements per
@@ -1959,6 +1983,10 @@ void plan_local(heomgb_qme_solver* qs) {
   qs->local = true;
 }
 
+ClusterForm cluster_form(const heomgb_qme_solver* qs) {
+  return qs->mixed ? kClusterMixed : qs->rotated ? kClusterFp64Comp : kClusterFp64;
+}
+
 // Cluster-resident fixed steps (k_cluster) apply to RK4 and LSRK4 on the
 // diagonal-coupling path without a terminator when the bins fit the clusters'
 // shared memory.  For every cluster size, as many bins as clusters are resident
@@ -1986,6 +2014,7 @@ void plan_cluster(heomgb_qme_solver* qs) {
   if (const char* env = std::getenv("HEOMGB_CLUSTER_SIZE")) pin_size = std::atoi(env);
   const std::vector<DiagInst>& insts = qs->plan.inst;
   const bool mixed = qs->mixed;
+  const ClusterForm form = cluster_form(qs);
   const int scheme = resident_scheme(qs);
   int terms = 1;
   for (const DiagInst& I : insts) {
@@ -2006,7 +2035,7 @@ void plan_cluster(heomgb_qme_solver* qs) {
   for (int size = 1; size <= kClusterMaxSize; size *= 2) {
     if (pin_size && size != pin_size) continue;
     // clusters resident at once (a cluster's CTAs share a GPC, so not every SM gets one)
-    const int active = cluster_active(mixed, scheme, 1, size, kClusterMaxBlock, 200 * 1024);
+    const int active = cluster_active(form, scheme, 1, size, kClusterMaxBlock, 200 * 1024);
     if (active < 1) continue;
     const int want = static_cast<int>(std::min<size_t>(insts.size(), static_cast<size_t>(active)));
     std::vector<long long> load(want, 0);
@@ -2058,7 +2087,7 @@ void plan_cluster(heomgb_qme_solver* qs) {
       sh.ept = ept;
       sh.block = std::max(32, ((lanes + ept - 1) / ept + 31) / 32 * 32);
       if (sh.block > (ept > 2 ? 512 : kClusterMaxBlock)) continue;
-      if (cluster_active(mixed, scheme, ept, size, sh.block, sh.smem) >= 1) shapes.push_back(sh);
+      if (cluster_active(form, scheme, ept, size, sh.block, sh.smem) >= 1) shapes.push_back(sh);
       break;
     }
   }
@@ -2087,7 +2116,7 @@ void plan_cluster(heomgb_qme_solver* qs) {
     for (int r = 0; r < 4; ++r) {  // best of two
       a.n_steps = (r & 1) ? 11 : 3;
       ck(cudaEventRecord(e0, qs->stream), "event");
-      ck(launch_cluster(a, mixed, scheme, sh.ept, sh.size, sh.bins, sh.block, sh.smem, qs->stream), "cluster tune");
+      ck(launch_cluster(a, form, scheme, sh.ept, sh.size, sh.bins, sh.block, sh.smem, qs->stream), "cluster tune");
       ck(cudaEventRecord(e1, qs->stream), "event");
       ck(cudaEventSynchronize(e1), "event sync");
       float ms = 0.f;
@@ -2105,7 +2134,7 @@ void plan_cluster(heomgb_qme_solver* qs) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  const float rival = qs->local ? qs->loc_step_ms : qs->resident ? qs->res_step_ms : 4.f * qs->stage_ms;
+  const float rival = qs->rotated ? 1e30f : qs->local ? qs->loc_step_ms : qs->resident ? qs->res_step_ms : 4.f * qs->stage_ms;
   if (!force && !(best_ms < rival)) return;
   const Shape& sh = shapes[best];
   qs->clu.inst = qs->plan.ds.inst;
@@ -2293,7 +2322,7 @@ void solve_fixed(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwarg
     a.dt_step = dt;
     a.dt_last = last;
     busy_begin(qs);
-    ck(launch_cluster(a, qs->mixed, resident_scheme(qs), qs->clu_ept, qs->clu_size, qs->clu_bins, qs->clu_block,
+    ck(launch_cluster(a, cluster_form(qs), resident_scheme(qs), qs->clu_ept, qs->clu_size, qs->clu_bins, qs->clu_block,
                       qs->clu_smem, qs->stream),
        "cluster-resident interval");
     busy_end(qs);
@@ -2493,7 +2522,7 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
     if (i == 0 || cb) {
       if (qs->rotated) {
         ck(cudaMemcpyAsync(qs->otmp, rho, bytes, in_kind, qs->stream), "state in");
-        ck(launch_rotate(qs->otmp, qs->S[0], qs->q->rbasis, qs->q->n, qs->q->n_hrchy, true, qs->col_major, false,
+        ck(launch_rotate(qs->otmp, qs->S[0], qs->q->rbasis, qs->q->rbasis_lo, qs->q->n, qs->q->n_hrchy, true, qs->col_major, false,
                          qs->stream),
            "rotate in");
       } else if (qs->col_major) {  // the caller's ADOs are column-major: transpose at the boundary
@@ -2511,7 +2540,7 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
     else
       solve_fixed(qs, t_list[i], t_list[i + 1], kw);
     if (qs->rotated) {
-      ck(launch_rotate(qs->S[cur], qs->otmp, qs->q->rbasis, qs->q->n, qs->q->n_hrchy, false, false, qs->col_major,
+      ck(launch_rotate(qs->S[cur], qs->otmp, qs->q->rbasis, qs->q->rbasis_lo, qs->q->n, qs->q->n_hrchy, false, false, qs->col_major,
                        qs->stream),
          "rotate out");
       ck(cudaMemcpyAsync(rho, qs->otmp, bytes, out_kind, qs->stream), "state out");

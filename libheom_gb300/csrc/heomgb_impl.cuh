@@ -276,11 +276,13 @@ struct ClusterArgs {
   int ecap;                 // elements of the fullest CTA
   int terms;                // bath-term slots per element
 };
+// the mixed form, FP64, FP64 with the state's rounding errors carried along
+enum ClusterForm { kClusterMixed, kClusterFp64, kClusterFp64Comp };
 int cluster_lanes(bool mixed);  // lanes per element
 int cluster_elements(const int* n2, const int* nh, int count, int size);  // of a bin's fullest CTA
 size_t cluster_smem(int h_elems, int ecap, int terms, bool mixed);
-int cluster_active(bool mixed, int scheme, int ept, int size, int block, size_t smem);
-cudaError_t launch_cluster(const ClusterArgs& args, bool mixed, int scheme, int ept, int size, int bins, int block,
+int cluster_active(ClusterForm form, int scheme, int ept, int size, int block, size_t smem);
+cudaError_t launch_cluster(const ClusterArgs& args, ClusterForm form, int scheme, int ept, int size, int bins, int block,
                            size_t smem, cudaStream_t s);
 
 // Lifts a kernel's limits to the device's: dynamic shared memory, and (largest) the
@@ -339,9 +341,11 @@ cudaError_t launch_scaled_coef(int n_terms, int rows, const double2* c, double2*
                                cudaStream_t s);
 cudaError_t launch_transpose_ados(const double2* in, double2* out, int n, long long count, cudaStream_t s);
 // `count` n x n blocks into (W^dagger X W) or out of (W X W^dagger) the basis W (row-major,
-// a column per basis vector); in_t, out_t: blocks stored column-major on that side.  Out of place.
-cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, int n, long long count, bool into,
-                          bool in_t, bool out_t, cudaStream_t s);
+// a column per basis vector; W + Wl to twice the FP64 precision, the results rounded
+// once); in_t, out_t: blocks stored column-major on that side.  Out of place.
+constexpr int kRotateMaxN = 32;
+cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, const double2* Wl, int n, long long count,
+                          bool into, bool in_t, bool out_t, cudaStream_t s);
 cudaError_t launch_ctl_init(DpCtl* c, double t, double dt, double t_bound, double atol, double rtol, int cur,
                             cudaStream_t s);
 cudaError_t launch_ctl_set_fixed(DpCtl* c, double dt, cudaStream_t s);

@@ -2315,22 +2315,40 @@ cudaError_t launch_transpose_ados(const double2* in, double2* out, int n, long l
   return cudaGetLastError();
 }
 
+// Sums of products in twice the FP64 precision: s + c += a b, with a = (h, l).
+__device__ __forceinline__ void add_wide(double& s, double& c, double ah, double al, double bh, double bl) {
+  const double p = __dmul_rn(ah, bh), e = fma(ah, bl, fma(al, bh, fma(ah, bh, -p)));
+  const double t = __dadd_rn(s, p), z = __dsub_rn(t, s);
+  c = __dadd_rn(c, __dadd_rn(__dadd_rn(__dsub_rn(s, __dsub_rn(t, z)), __dsub_rn(p, z)), e));
+  s = t;
+}
+__device__ __forceinline__ void cadd_wide(double2& s, double2& c, double2 ah, double2 al, double2 bh, double2 bl) {
+  add_wide(s.x, c.x, ah.x, al.x, bh.x, bl.x);
+  add_wide(s.x, c.x, -ah.y, -al.y, bh.y, bl.y);
+  add_wide(s.y, c.y, ah.x, al.x, bh.y, bl.y);
+  add_wide(s.y, c.y, ah.y, al.y, bh.x, bl.x);
+}
+
 // A CTA takes `per` blocks at a time: the blocks and W in shared memory, the
-// left product beside them, the right product on the way out.  Runs twice a
-// solve, beside the copies of the state.
+// left product beside them, the right product on the way out, both in twice
+// the FP64 precision (about 30 FP64 operations a real product).  Runs twice a
+// solve or interval, beside the copies of the state: 286 blocks of 2 x 2 take a few us.
 __global__ void __launch_bounds__(256) k_rotate(const double2* __restrict__ in, double2* __restrict__ out,
-                                                const double2* __restrict__ W, int n, long long count, int per,
-                                                int into, int in_t, int out_t) {
+                                                const double2* __restrict__ W, const double2* __restrict__ Wl, int n,
+                                                long long count, int per, int into, int in_t, int out_t) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n2 = n * n;
-  double2* Ws = reinterpret_cast<double2*>(smem_raw);
-  double2* X = Ws + n2;
-  double2* T = X + static_cast<size_t>(per) * n2;
+  double2* Ah = reinterpret_cast<double2*>(smem_raw);
+  double2* Al = Ah + n2;
+  double2* X = Al + n2;
+  double2* Th = X + static_cast<size_t>(per) * n2;
+  double2* Tl = Th + static_cast<size_t>(per) * n2;
   // A = W^dagger (into) or W: T = A X, out = T A^dagger
   for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-    const int a = i / n, b = i - a * n;
-    const double2 w = into ? W[b * n + a] : W[i];
-    Ws[i] = make_double2(w.x, into ? -w.y : w.y);
+    const int a = i / n, b = i - a * n, j = into ? b * n + a : i;
+    const double sg = into ? -1.0 : 1.0;
+    Ah[i] = make_double2(W[j].x, sg * W[j].y);
+    Al[i] = make_double2(Wl[j].x, sg * Wl[j].y);
   }
   for (long long l0 = static_cast<long long>(blockIdx.x) * per; l0 < count; l0 += static_cast<long long>(gridDim.x) * per) {
     const int ne = static_cast<int>(min(static_cast<long long>(per), count - l0)) * n2;
@@ -2342,35 +2360,38 @@ __global__ void __launch_bounds__(256) k_rotate(const double2* __restrict__ in, 
     __syncthreads();
     for (int i = threadIdx.x; i < ne; i += blockDim.x) {
       const int lt = i / n2, e = i - lt * n2, a = e / n, b = e - a * n;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = 0; c < n; ++c) cfma(acc, Ws[a * n + c], X[lt * n2 + c * n + b]);
-      T[i] = acc;
+      double2 s = make_double2(0.0, 0.0), c = s;
+      for (int k = 0; k < n; ++k)
+        cadd_wide(s, c, Ah[a * n + k], Al[a * n + k], X[lt * n2 + k * n + b], make_double2(0.0, 0.0));
+      Th[i] = s;
+      Tl[i] = c;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < ne; i += blockDim.x) {
       const int lt = i / n2, e = i - lt * n2;
       const int a = out_t ? e % n : e / n, b = out_t ? e / n : e % n;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = 0; c < n; ++c) {
-        const double2 w = Ws[b * n + c];
-        cfma(acc, T[lt * n2 + a * n + c], make_double2(w.x, -w.y));
+      double2 s = make_double2(0.0, 0.0), c = s;
+      for (int k = 0; k < n; ++k) {
+        const double2 wh = Ah[b * n + k], wl = Al[b * n + k];
+        cadd_wide(s, c, Th[lt * n2 + a * n + k], Tl[lt * n2 + a * n + k], make_double2(wh.x, -wh.y),
+                  make_double2(wl.x, -wl.y));
       }
-      out[l0 * n2 + i] = acc;
+      out[l0 * n2 + i] = make_double2(s.x + c.x, s.y + c.y);
     }
   }
 }
 
-cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, int n, long long count, bool into,
-                          bool in_t, bool out_t, cudaStream_t s) {
+cudaError_t launch_rotate(const double2* in, double2* out, const double2* W, const double2* Wl, int n, long long count,
+                          bool into, bool in_t, bool out_t, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   const int n2 = n * n, per = std::max(1, 256 / n2);
-  const size_t smem = sizeof(double2) * static_cast<size_t>(n2) * (1 + 2 * per);
+  const size_t smem = sizeof(double2) * static_cast<size_t>(n2) * (2 + 3 * per);
   if (smem > 48 * 1024) {
     cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_rotate));
     if (e != cudaSuccess) return e;
   }
   const int grid = static_cast<int>(std::min<long long>((count + per - 1) / per, 152 * 8));
-  k_rotate<<<grid, 256, smem, s>>>(in, out, W, n, count, per, into ? 1 : 0, in_t ? 1 : 0, out_t ? 1 : 0);
+  k_rotate<<<grid, 256, smem, s>>>(in, out, W, Wl, n, count, per, into ? 1 : 0, in_t ? 1 : 0, out_t ? 1 : 0);
   ++g_launches;
   return cudaGetLastError();
 }

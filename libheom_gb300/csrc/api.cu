@@ -500,6 +500,7 @@ struct heomgb_qme_solver {
   cudaGraphExec_t g_small = nullptr, g_big = nullptr;
   int n_small = 0, n_big = 0;           // steps (fixed) or attempts (DP) per graph
   int nodes_small = 0, nodes_big = 0;
+  bool refit = false;  // a resident plan did not fit after all: the next solve searches the stage kernels' shape
   double dt_save = -1.0;
   long long n_rhs = 0, n_attempts = 0, n_accepted = 0;
   // device time spent inside graph replays of the last solve (CUDA events on
@@ -1364,6 +1365,14 @@ ResidentArgs resident_args(heomgb_qme_solver* qs) {
     a.spin_limit = std::max(1LL, std::min(1LL << 24, std::atoll(env)));
   return a;
 }
+// One resident interval.  HEOMGB_FAULT_COOPERATIVE=1 answers as a device that cannot
+// hold the grid does, for the tests of that way out.
+cudaError_t launch_interval(heomgb_qme_solver* qs, const ResidentArgs& a) {
+  if (const char* env = std::getenv("HEOMGB_FAULT_COOPERATIVE"))
+    if (std::string(env) == "1") return cudaErrorCooperativeLaunchTooLarge;
+  return launch_resident(a, resident_variant(qs), solver_inst(qs).h_real != 0, qs->res_ept, qs->res_grid, qs->res_block,
+                         qs->res_smem, qs->stream);
+}
 Stage solver_stage(heomgb_qme_solver* qs);
 
 // The diagonal-coupling instances of the solver's models, concatenated.
@@ -1419,7 +1428,7 @@ void alloc_solver(heomgb_qme_solver* qs) {
   if (plan_rotated(qs)) return;
   // a model that runs as resident intervals needs no tile search: its stage
   // kernels (the fall-back, should the device not hold the cooperative grid) take
-  // the default shape
+  // the default shape until the next solve (refit)
   if (!std::getenv("HEOMGB_TILE")) plan_resident(qs);
   if (qs->path == PATH_DIAG) {
     if (qs->resident)
@@ -2360,8 +2369,7 @@ void solve_fixed(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwarg
     a.dt_step = dt;
     a.dt_last = last;
     busy_begin(qs);
-    const cudaError_t le = launch_resident(a, resident_variant(qs), solver_inst(qs).h_real != 0, qs->res_ept,
-                                           qs->res_grid, qs->res_block, qs->res_smem, qs->stream);
+    const cudaError_t le = launch_interval(qs, a);
     if (le != cudaErrorCooperativeLaunchTooLarge) {
       ck(le, "resident interval");
       busy_end(qs);
@@ -2379,6 +2387,7 @@ void solve_fixed(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwarg
     }
     // the device cannot hold the grid now: this and later intervals take the graphs
     cudaGetLastError();
+    qs->refit = true;
     busy_end(qs);
     ck(cudaStreamSynchronize(qs->stream), "solve sync");
     busy_collect(qs);
@@ -2416,12 +2425,12 @@ int solve_resident(heomgb_qme_solver* qs, double t0, double t1, const heomgb_kwa
   ck(launch_ctl_init(qs->ctl, t0, dt, t1, atol, rtol, cur, qs->stream), "ctl init");
   ck(cudaMemsetAsync(qs->res_bar, 0, kResidentBarWords * sizeof(unsigned long long), qs->stream), "barrier reset");
   busy_begin(qs);
-  const cudaError_t le = launch_resident(resident_args(qs), resident_variant(qs), solver_inst(qs).h_real != 0, qs->res_ept,
-                                         qs->res_grid, qs->res_block, qs->res_smem, qs->stream);
+  const cudaError_t le = launch_interval(qs, resident_args(qs));
   if (le == cudaErrorCooperativeLaunchTooLarge) {
     // the device cannot hold the grid now (another context holds SMs or
     // shared memory): this and later intervals take the stage kernels
     cudaGetLastError();
+    qs->refit = true;
     busy_end(qs);
     ck(cudaStreamSynchronize(qs->stream), "solve sync");
     busy_collect(qs);
@@ -2491,6 +2500,22 @@ void transpose_instances(heomgb_qme_solver* qs, const double2* in, double2* out)
   }
 }
 
+// The stage kernels' tile search, for a solver whose resident plan the device
+// refused (alloc_solver gave its stage kernels the default shape, and the solve that
+// met the refusal ended on it: the search needs the state's buffers).
+void refit(heomgb_qme_solver* qs) {
+  qs->refit = false;
+  autotune(qs);
+  qs->block = qs->plan.block;
+  if (qs->plan.grid > qs->grid)
+    qs->partials = static_cast<double*>(qs->arena.alloc(sizeof(double) * qs->plan.grid));
+  qs->grid = qs->plan.grid;
+  for (cudaGraphExec_t* g : {&qs->g_small, &qs->g_big}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+}
+
 void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_list, int n_t, heomgb_callback cb,
                 void* user, const heomgb_kwargs* kw) {
   const NvtxRange range("heomgb solve");
@@ -2503,6 +2528,7 @@ void solve_impl(heomgb_qme_solver* qs, void* rho, bool host, const double* t_lis
     ck(cudaEventRecord(qs->user_ready, qs->q->stream()), "event record");
     ck(cudaStreamWaitEvent(qs->stream, qs->user_ready, 0), "stream wait");
   }
+  if (qs->refit) refit(qs);
   qs->n_rhs = qs->n_attempts = qs->n_accepted = 0;
   qs->busy_ms = 0.0;
   qs->replayed_kernels = 0;

@@ -887,7 +887,6 @@ DiagInst make_diag_inst(heomgb_qme* q, const std::vector<cd>& H, const std::vect
       const int* dms = q->arena.upload(msite, s);
       di.site_cm3 = q->arena.upload(to_f2(cm3), s);
       di.site_cp2 = q->arena.upload(to_f2(cp2), s);
-      di.site_cm3_d = q->arena.upload(to_d2(cm3), s);
       di.site_cp2_d = q->arena.upload(to_d2(cp2), s);
       di.site_ptr = q->arena.upload(sptr, s);
       di.site_modes = q->arena.upload(smodes, s);

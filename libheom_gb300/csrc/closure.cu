@@ -1,5 +1,5 @@
 // The learned closure's fused tensor-core kernels: the inference of one stage
-// (k_term_mlp) and the training pass over a minibatch (k_train, k_dw, k_finish).
+// (k_term_mlp) and the training pass over a minibatch (k_train, k_dw, k_adam).
 //
 // A CTA keeps the activations of its tile of rows in shared memory as BF16
 // core matrices and the accumulators in tensor memory.  The weights come
@@ -308,7 +308,7 @@ __global__ void k_term_tables(const TermModel tm, int first, int n_tier, float2*
 // weight gradient D^T = X^T dZ (inputs along the tensor-memory lanes, so a
 // warp stores 32 consecutive entries of a row of dW) and runs through the
 // rows in order in one accumulator: the summation order of the GEMM over the
-// whole batch, whatever the number of tiles.  k_finish: Adam.
+// whole batch, whatever the number of tiles.  k_adam: Adam.
 //
 // BF16 rounding happens where the operands are written instead of where a
 // GEMM reads them: the same values, and every sum (MMAs over the rows in

@@ -165,9 +165,8 @@ struct DiagInst {
   const float2* site_cp2;   // K * 2: the +1 coefficient of mode k in its site's row / column
   const int* site_ptr;      // n + 1: the modes of site s are site_modes[site_ptr[s] .. site_ptr[s+1])
   const int* site_modes;    // K, per site in increasing k
-  const double2* site_cm3_d;  // K * 3 and K * 2: the same coefficients in FP64 (the FP64 resident interval)
-  const double2* site_cp2_d;
-  const double2* site_cmn_d;  // site_cm3_d scaled by the occupation: row (3 k + case) * occ_rows + n_k
+  const double2* site_cp2_d;  // K * 2: site_cp2 in FP64 (k_dp_resident64, k_rhs_split)
+  const double2* site_cmn_d;  // site_cm3 in FP64, scaled by the occupation: row (3 k + case) * occ_rows + n_k
   // k_rhs_split (FP64, real symmetric H): H's digits as its B operand, and the exponents of its columns' scales
   const uint4* h_digits;
   const int* h_exp;

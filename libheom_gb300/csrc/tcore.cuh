@@ -1,6 +1,7 @@
-// PTX wrappers of the tensor-core kernels of the learned closure: descriptors
-// and issue of tcgen05.mma (kind::f16, BF16 operands, FP32 accumulators in
-// tensor memory), tensor-memory loads, bulk copies and bounded mbarrier waits.
+// PTX wrappers of the 16-bit tensor-core kernels (the learned closure's and its
+// GEMMs, BF16; k_rhs_split, FP16): descriptors and issue of tcgen05.mma
+// (kind::f16, FP32 accumulators in tensor memory), tensor-memory loads, bulk
+// copies and bounded mbarrier waits.
 #pragma once
 
 #include <cuda_bf16.h>

@@ -233,8 +233,9 @@ heomgb_status heomgb_qme_solver_resident(const heomgb_qme_solver* qs, int* on, i
 heomgb_status heomgb_qme_solver_row_kernel(const heomgb_qme_solver* qs, int* on);
 /* 1 when the solver's FP64 stages compute the commutator on the tensor cores
  * from exact digits (site-local baths, real symmetric H, 4 to 32 levels).
- * Taken by a rule on sizes; HEOMGB_SPLIT=0 keeps it out, =1 takes it wherever it
- * can run.  No reference counterpart. */
+ * An element's error bound is no larger than with FP64 sums, its roundings are
+ * others.  Taken by a rule on sizes; HEOMGB_SPLIT=0 keeps it out, =1 takes it
+ * wherever it can run.  No reference counterpart. */
 heomgb_status heomgb_qme_solver_split(const heomgb_qme_solver* qs, int* on);
 /* Whether fixed steps run as cluster-resident intervals (one launch per output
  * interval, a thread-block cluster of `size` CTAs of `block` threads per bin of

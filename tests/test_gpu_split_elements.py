@@ -100,3 +100,69 @@ def test_zero_columns_and_zero_parts(n, monkeypatch):
     ref = oracle.Oracle("port").solve(p, rho.copy(), [0.0, 3.7, 10.0], solver="rk4", dt=dt)[-1]
     got = solve([p], "rk4", rho.copy(), "1", monkeypatch)
     assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+def _model(r):
+    """A commutator alone (depth 0) with H and the state of one of several shapes."""
+    n = int(r.integers(4, 33))
+    p = configs.aggregate_24site(n_sites=n, depth=0, seed=int(r.integers(1000)))
+    H, kind = p.H.real.copy(), int(r.integers(6))
+    if kind == 1:
+        H = np.diag(np.diag(H)) + np.diag(np.full(n - 1, 0.01), 1) + np.diag(np.full(n - 1, 0.01), -1)
+    elif kind == 2:  # columns over 12 decades
+        g = 10.0 ** r.uniform(-12, 0, n)
+        H = H * (g[:, None] * g[None, :])
+    elif kind == 3:  # few couplings
+        m = np.triu(r.uniform(size=(n, n)) < 0.2, 1)
+        H = H * (m + m.T)
+    elif kind == 4:
+        H = H + np.eye(n) * r.uniform(-5, 5)
+    elif kind == 5:  # uncoupled sites of energy 0
+        z = r.uniform(size=n) < 0.3
+        H[z], H[:, z] = 0.0, 0.0
+    rho, kind = r.standard_normal((n, n)) + 1j * r.standard_normal((n, n)), int(r.integers(6))
+    if kind == 1:
+        g = 10.0 ** r.uniform(-30, 0, n)
+        rho = rho * (g[:, None] * g[None, :])
+    elif kind == 2:
+        rho = rho * (r.uniform(size=(n, n)) < 0.15)
+    elif kind == 3:
+        rho = rho.real + 0j
+    elif kind == 4:
+        rho = rho * (10.0 ** r.uniform(-100, 100, (n, 1)) * 10.0 ** r.uniform(-100, 100, (1, n)))
+    elif kind == 5:
+        rho = rho * 10.0 ** r.uniform(-8, 0, (n, n))
+    return dataclasses.replace(p, H=H.astype(complex)), rho[None]
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_every_element_within_the_bound_of_fp64_sums(seed, monkeypatch):
+    """One RK4 step of a batch of commutators against numpy's longdouble.  An
+    element's bound: 2^-53 times the roundings of a chain of FP64 sums (2 n
+    products and 10 other operations a stage, 4 stages) times the step formed
+    with absolute values."""
+    r, dt = np.random.default_rng(seed), 0.05
+    models = [_model(r) for _ in range(30)]
+    monkeypatch.setattr("test_gpu_split.DT", dt)
+    flat = np.concatenate([rho.ravel() for _, rho in models])
+    got, o = solve([p for p, _ in models], "rk4", flat, "1", monkeypatch, (0.0, dt)), 0
+    for p, rho in models:
+        n = p.n_level
+        sd = np.zeros((n, n), complex)
+        for u in range(p.n_noise):
+            v = np.diag(p.V[u])
+            sd += p.s_delta[u] * (v[:, None] - v[None, :]) ** 2
+
+        def step(H, s, y, f):
+            k1 = f(H, s, y)
+            k2 = f(H, s, y + k1 / 2)
+            k3 = f(H, s, y + k2 / 2)
+            return y + (k1 + 2 * k2 + 2 * k3 + f(H, s, y + k3)) / 6
+
+        C, h = np.clongdouble, np.longdouble(dt)
+        want = step(p.H.astype(C), sd.astype(C), rho[0].astype(C), lambda H, s, x: -h * (C(1j) * (H @ x - x @ H) + s * x))
+        bound = step(np.abs(p.H), np.abs(sd), np.abs(rho[0].real) + np.abs(rho[0].imag),
+                     lambda H, s, x: dt * (H @ x + x @ H + s * x))
+        err = np.abs((got[o:o + n * n].reshape(n, n) - want).astype(complex))
+        assert (err <= 2.0**-53 * 4 * (2 * n + 10) * bound + 1e-300).all()
+        o += n * n

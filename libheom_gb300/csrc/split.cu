@@ -23,10 +23,10 @@
 // localised on a chain), rows whose largest value lies outside 2^-800 .. 2^900,
 // infinities and NaNs take FP64 sums in pass 5.  One scale for an ADO and seven
 // digits were faster (0.59 ms where this takes 0.78) and lost the small elements of
-// graded states.  Measured against 64 bits, four steps of 24 sites: 7.5e-17 of
-// the state's norm, as with FP64 sums.  A stage of the 24-site model at depth 3
-// (12M elements) takes 0.78 ms, 2.95 with k_rhs_diag<double>, whose FP64 pipe alone
-// needs 2.58 (16 sites: 0.115 and 0.287).
+// graded states.  Measured against 64 bits, 24 sites, mean of eight states: 8.1e-17
+// of the norm after four steps (FP64 sums 9.7e-17), 3.0e-16 after 40 (3.4e-16).  A
+// stage of the 24-site model at depth 3 (12M elements) takes 0.78 ms, 2.95 with
+// k_rhs_diag<double>, whose FP64 pipe alone needs 2.58 (16 sites: 0.115 and 0.287).
 //
 // Per tile of T = 128 / (4 n) ADOs, the first group of a CTA (256 threads):
 //   1. the stage input (copied with cp.async a tile ahead), the largest exponent
